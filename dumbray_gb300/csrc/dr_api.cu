@@ -477,7 +477,7 @@ dr_status dr_scene_create(const float *xyz, const float *nrm, const int32_t *mat
 
     std::vector<float> gbox, gbox_ref;
     group_planes(T, gbox, gbox_ref);
-    float4 *d_nodes = nullptr, *d_gbox = nullptr, *d_gbox_ref = nullptr, *d_leaf = nullptr, *d_tris = nullptr, *d_nrms = nullptr;
+    float4 *d_nodes = nullptr, *d_gbox = nullptr, *d_gbox_ref = nullptr, *d_groups = nullptr, *d_leaf = nullptr, *d_tris = nullptr, *d_nrms = nullptr;
     int *d_mat = nullptr;
     drd::Material *d_mats = nullptr;
     drd::Light *d_lights = nullptr;
@@ -491,6 +491,15 @@ dr_status dr_scene_create(const float *xyz, const float *nrm, const int32_t *mat
     if (e == cudaSuccess) { sc->allocs.push_back(d_mat); e = upload(&d_mats, dm.data(), dm.size()); }
     if (e == cudaSuccess) { sc->allocs.push_back(d_mats); e = upload(&d_lights, dl.data(), dl.size()); }
     if (e == cudaSuccess) sc->allocs.push_back(d_lights);
+    float reach = 0.0f;
+    for (int k = 0; k < 3; k++) reach = std::fmax(reach, std::fmax(std::fabs(T.root_lo[k]), std::fabs(T.root_hi[k])));
+    const int64_t n_groups = T.node_count / 8;
+    if (e == cudaSuccess && n_groups) e = cudaMalloc((void **)&d_groups, sizeof(float4) * drd::kRecordF4 * (size_t)n_groups);
+    if (e == cudaSuccess && n_groups) {
+        sc->allocs.push_back(d_groups);
+        e = drk::launch_group_records(d_groups, d_nodes, d_gbox, n_groups, reach * drd::kRecordPad, nullptr);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+    }
     if (e != cudaSuccess) {
         delete sc;
         return cuda_fail(e, "dr_scene_create: upload");
@@ -501,6 +510,8 @@ dr_status dr_scene_create(const float *xyz, const float *nrm, const int32_t *mat
     S.nodes = d_nodes;
     S.gbox = d_gbox;
     S.gbox_ref = d_gbox_ref;
+    S.groups = d_groups;
+    S.reach = reach;
     S.leaf_tris = d_leaf;
     S.tris = d_tris;
     S.nrms = d_nrms;
@@ -1146,7 +1157,7 @@ struct dr_batch {
     cudaEvent_t done = nullptr;   // recorded after each render: the job table is in use until it fires
     // One device arena holding the octrees of all the batch's scenes (node child / leaf indices
     // rebased), so the traversal reads nodes and leaf triangles through one pointer for every ray.
-    float4 *arena_nodes = nullptr, *arena_gbox = nullptr, *arena_leaf = nullptr;
+    float4 *arena_nodes = nullptr, *arena_gbox = nullptr, *arena_groups = nullptr, *arena_leaf = nullptr;
     int64_t arena_node_count = 0;
 
     void drop_graph() {
@@ -1162,6 +1173,7 @@ struct dr_batch {
         if (done) cudaEventDestroy(done);
         cudaFree(arena_nodes);
         cudaFree(arena_gbox);
+        cudaFree(arena_groups);
         cudaFree(arena_leaf);
         cudaFree(items_dev);
     }
@@ -1191,6 +1203,8 @@ static dr_status build_arena(dr_batch *b) {
     cudaError_t e = cudaMalloc((void **)&b->arena_nodes, sizeof(float4) * (size_t)std::max<int64_t>(nodes, 2));
     if (e == cudaSuccess) e = cudaMalloc((void **)&b->arena_leaf, sizeof(float4) * (size_t)std::max<int64_t>(leaf, 3));
     if (e == cudaSuccess) e = cudaMalloc((void **)&b->arena_gbox, sizeof(float4) * 12 * (size_t)std::max<int64_t>(nodes / 16, 1));
+    if (e == cudaSuccess)
+        e = cudaMalloc((void **)&b->arena_groups, sizeof(float4) * drd::kRecordF4 * (size_t)std::max<int64_t>(nodes / 16, 1));
     for (size_t k = 0; k < uniq.size() && e == cudaSuccess; k++) {
         const dr_scene *sc = uniq[k];
         if (sc->leaf_f4)
@@ -1202,6 +1216,9 @@ static dr_status build_arena(dr_batch *b) {
         if (e == cudaSuccess && sc->node_f4)
             e = drk::launch_rebase_nodes(b->arena_nodes + 2 * node_off[k], sc->dev.nodes, sc->node_f4 / 2, (int)(node_off[k] / 8),
                                          (int)leaf_off[k], nullptr);
+        if (e == cudaSuccess && sc->node_f4)
+            e = drk::launch_rebase_groups(b->arena_groups + drd::kRecordF4 * (node_off[k] / 8), sc->dev.groups, sc->node_f4 / 16,
+                                          (int)(node_off[k] / 8), (int)leaf_off[k], nullptr);
     }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return cuda_fail(e, "dr_batch_create: octree arena");
@@ -1215,6 +1232,7 @@ static dr_status build_arena(dr_batch *b) {
         drd::Scene &S = b->items[i].S;
         S.nodes = b->arena_nodes;
         S.gbox = b->arena_gbox;
+        S.groups = b->arena_groups;
         S.gbox_ref = b->arena_gbox;   // batches do not run the counting traversal
         S.leaf_tris = b->arena_leaf;
         if (S.root_child >= 0) S.root_child += (int)(node_off[k] / 8);

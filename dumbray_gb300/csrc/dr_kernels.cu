@@ -150,6 +150,7 @@ struct BatchSource {
         job = 0;
         return true;
     }
+    __device__ __forceinline__ int job(int) { return 0; }
     // single-scene source: never asked for a per-job scene (MULTI = false)
     __device__ __forceinline__ const Scene &scene(int) { return *scene0; }
     __device__ __forceinline__ bool clip(int) { return cull; }
@@ -168,7 +169,7 @@ template <bool COUNT>
 __global__ void __launch_bounds__(128) k_cast(Scene S, const float *__restrict__ o, const float *__restrict__ d,
                                               const int *__restrict__ ignore, int n, int clip, int *__restrict__ hit_tri,
                                               float *__restrict__ hit_t, int *__restrict__ nbox, int *__restrict__ ntri) {
-    uint32_t stack[kStack];
+    typename StackOf<COUNT>::type stack[kStack];
     __shared__ WarpLeafSlots slots[4];
     BatchSource src{o, d, ignore, hit_tri, COUNT ? nbox : nullptr, COUNT ? ntri : nullptr, hit_t, n, false, clip != 0, &S};
     trace_persistent<COUNT, false>(S, src, stack, slots[threadIdx.x >> 5]);
@@ -382,6 +383,7 @@ struct TraceSource {
         job = p3.w;
         return true;
     }
+    __device__ __forceinline__ int job(int i) { return Q.p3[i].w; }
     __device__ __forceinline__ const Scene &scene(int job) { return job_of<MULTI>(*A, job).S; }
     __device__ __forceinline__ bool clip(int job) {
         const Item &I = job_of<MULTI>(*A, job);
@@ -409,7 +411,7 @@ template <bool COUNT, bool MULTI, int TT = kTraceThreads, int TB = kTraceBlocksP
 __global__ void __launch_bounds__(TT, TB) k_trace(WaveArgs A, int b) {
     Ctrl *C = A.ctrl;
     const int n = *((volatile int *)&C->ray_count[b]);
-    uint32_t stack[kStack];
+    typename StackOf<COUNT>::type stack[kStack];
     __shared__ WarpLeafSlots slots[TT / 32];
     TraceSource<MULTI> src{&A, A.q[b & 1], A.hits, &C->fetch_trace[b], n, chunk_for(n), 0, 0, 0};
     trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], A.inl.S.front_only ? kPhysStepsPerRound : 1);
@@ -600,6 +602,7 @@ struct RefPhotonSource {
         job = __float_as_int(sq.s4[i].w);
         return true;
     }
+    __device__ __forceinline__ int job(int i) { return __float_as_int(sq.s4[i].w); }
     __device__ __forceinline__ const Scene &scene(int job) { return job_of<MULTI>(*A, job).S; }
     __device__ __forceinline__ bool clip(int job) { return job_of<MULTI>(*A, job).clip != 0; }
     __device__ __forceinline__ bool store(int i, const Hit &h, int b_, int t_) {
@@ -658,6 +661,7 @@ struct RefPhotonChainSource {
         job = __float_as_int(sq.s4[j].w);
         return true;
     }
+    __device__ __forceinline__ int job(int i) { return __float_as_int(sq.s4[blocked ? blocked[i] : i].w); }
     __device__ __forceinline__ const Scene &scene(int job) { return job_of<MULTI>(*A, job).S; }
     __device__ __forceinline__ bool clip(int job) { return job_of<MULTI>(*A, job).clip != 0; }
     __device__ __forceinline__ bool store(int i, const Hit &h, int b_, int t_) {
@@ -687,7 +691,7 @@ __global__ void __launch_bounds__(kTraceThreads, kShadowRefBlocksPerSM) k_shadow
     Ctrl *C = A.ctrl;
     const int n = *((volatile int *)&C->shadow_count[b]);
     if (n == 0) return;
-    uint32_t stack[kStack];
+    typename StackOf<COUNT>::type stack[kStack];
     __shared__ WarpLeafSlots slots[kTraceThreads / 32];
     RefPhotonSource<MULTI> src{&A, A.sq, &C->fetch_shadow[b], &C->carry_count, blocked_list(A, b), &C->blocked_count[b], n,
                                chunk_for(n), 0, 0, 0};
@@ -703,7 +707,7 @@ __global__ void __launch_bounds__(kTraceThreads, kPhotonChainBlocksPerSM) k_phot
     const bool carry = b < 0;
     const int n = carry ? min(*((volatile int *)&C->carry_count), A.carry_cap) : *((volatile int *)&C->blocked_count[b]);
     if (n == 0) return;
-    uint32_t stack[kStack];
+    typename StackOf<COUNT>::type stack[kStack];
     __shared__ WarpLeafSlots slots[kTraceThreads / 32];
     RefPhotonChainSource<MULTI> src{&A, carry ? A.cq : A.sq, carry ? nullptr : blocked_list(A, b),
                                     carry ? &C->fetch_carry : &C->fetch_chain[b], n, chunk_for(n), 0, 0, 0};
@@ -934,6 +938,7 @@ struct ShadowPhysSource {
         job = __float_as_int(sq.s4[i].w);
         return true;
     }
+    __device__ __forceinline__ int job(int i) { return __float_as_int(sq.s4[i].w); }
     __device__ __forceinline__ const Scene &scene(int job) { return job_of<MULTI>(*A, job).S; }
     __device__ __forceinline__ bool clip(int) { return false; }
     __device__ __forceinline__ bool store(int i, const Hit &h, int b_, int t_) {
@@ -986,7 +991,7 @@ template <bool COUNT, bool MULTI, bool ADJ, int TT = kTraceThreads, int TB = kTr
 __global__ void __launch_bounds__(TT, TB) k_shadow_phys(WaveArgs A, int b) {
     Ctrl *C = A.ctrl;
     const int n = *((volatile int *)&C->shadow_count[b]);
-    uint32_t stack[kStack];
+    typename StackOf<COUNT>::type stack[kStack];
     __shared__ WarpLeafSlots slots[TT / 32];
     ShadowPhysSource<MULTI, ADJ> src{&A, A.sq, A.accum, &C->fetch_shadow[b], n, chunk_for(n), 0, 0, 0};
     trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], A.inl.S.front_only ? kPhysStepsPerRound : 1);
@@ -1027,6 +1032,48 @@ __global__ void k_resolve(WaveArgs A, int total_slots) {
         float4 old = fb[at];
         fb[at] = make_float4((c.x * blend) + (old.x * (1.0f - blend)), (c.y * blend) + (old.y * (1.0f - blend)),
                              (c.z * blend) + (old.z * (1.0f - blend)), (c.w * blend) + (old.w * (1.0f - blend)));
+    }
+}
+
+// Group records (kRecordF4 layout) from the nodes and the refitted planes: one thread per word.
+__global__ void k_group_records(float *dst, const float4 *nodes, const float *gbox, long long n_groups, float pad) {
+    const long long n = n_groups * (4 * kRecordF4);
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const long long g = i / (4 * kRecordF4);
+        const int j = (int)(i - g * (4 * kRecordF4));
+        const float4 *node = nodes + 16 * g;
+        if (j < 48) {
+            const int axis = j >> 4, hi = (j >> 3) & 1, c = j & 7;
+            const float x = gbox[48 * g + 24 * hi + 8 * axis + c];
+            dst[i] = hi ? x + pad : x - pad;
+        } else if (j == 48) {
+            int links = 0;
+            for (int c = 7; c >= 0; c--) {
+                const int w = __float_as_int(node[2 * c].w);
+                if (w >= 0) links = ((w >> 3) << 8) | (links & 0xFF) | (1 << c);
+            }
+            dst[i] = __int_as_float(links);
+        } else {
+            // first reference of the first leaf child at or after j - 49, the end of the last one's past it
+            int at = 0;
+            bool found = false;
+            for (int c = 0; c < 8 && !found; c++) {
+                const int w = __float_as_int(node[2 * c].w);
+                if (w >= 0) continue;
+                at = c < j - 49 ? ~w + __float_as_int(node[2 * c + 1].w) : ~w;
+                found = c >= j - 49;
+            }
+            dst[i] = __int_as_float(at);
+        }
+    }
+}
+
+// Arena copy of one scene's group records: inner links += group_off, leaf references += leaf_off.
+__global__ void k_rebase_groups(uint32_t *dst, const uint32_t *src, long long n_groups, int group_off, int leaf_off) {
+    const long long n = n_groups * (4 * kRecordF4);
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const int j = (int)(i % (4 * kRecordF4));
+        dst[i] = src[i] + (j == 48 ? (uint32_t)group_off << 8 : j > 48 ? (uint32_t)leaf_off : 0u);
     }
 }
 
@@ -1282,6 +1329,24 @@ cudaError_t launch_rebase_nodes(float4 *dst, const float4 *src, long long n_node
     if (n_nodes <= 0) return cudaSuccess;
     const int grid = (int)std::min<long long>((n_nodes + 255) / 256, (long long)sm_count() * 8);
     drd::k_rebase_nodes<<<grid, 256, 0, stream>>>(dst, src, n_nodes, group_off, leaf_off);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_group_records(float4 *dst, const float4 *nodes, const float4 *gbox, long long n_groups, float pad,
+                                 cudaStream_t stream) {
+    if (n_groups <= 0) return cudaSuccess;
+    const int grid = (int)std::min<long long>((n_groups * 64 + 255) / 256, (long long)sm_count() * 32);
+    drd::k_group_records<<<grid, 256, 0, stream>>>(reinterpret_cast<float *>(dst), nodes, reinterpret_cast<const float *>(gbox),
+                                                   n_groups, pad);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_rebase_groups(float4 *dst, const float4 *src, long long n_groups, int group_off, int leaf_off,
+                                 cudaStream_t stream) {
+    if (n_groups <= 0) return cudaSuccess;
+    const int grid = (int)std::min<long long>((n_groups * 64 + 255) / 256, (long long)sm_count() * 32);
+    drd::k_rebase_groups<<<grid, 256, 0, stream>>>(reinterpret_cast<uint32_t *>(dst), reinterpret_cast<const uint32_t *>(src),
+                                                   n_groups, group_off, leaf_off);
     return cudaGetLastError();
 }
 

@@ -22,26 +22,39 @@ namespace drd {
 
 constexpr int kChunk = 256;
 
-enum : int { kIdle = 0, kTrav = 1, kLeaf = 2 };
+enum : int { kIdle = 0, kTrav = 1, kLeaf = 2, kDone = 3 };
 
 struct LaneRay {
-    f3 o, d, inv;
+    f3 o, d, inv;                    // inv: counting traversals
+    RaySlopes k;                     // every other traversal
     int order, ignore;
-    uint32_t cur;
+    uint32_t cur, links;             // group << shift | remaining hit mask; the group's word 48
     int sp;
     int r, r_end;
-    float lx, ly, lz, hx, hy, hz;
+    int node;                        // leaf node being tested, -1 = the root is the leaf
+    float lx, ly, lz, hx, hy, hz;    // its box (counting traversals)
     float best;
-    f3 bp;
-    int bi;
+    int pos;                         // list position of the nearest triangle so far
     int kleaf;
     int nb, nt;
+};
+
+// Stack entry of a traversal: the counting one packs the child position (see kCountShift), the others
+// keep the group's word 48 beside its index and remaining hit mask.
+template <bool COUNT>
+struct StackOf {
+    using type = uint2;
+};
+template <>
+struct StackOf<true> {
+    using type = uint32_t;
 };
 
 // Starts a ray: root leaf, root miss, or the root's children tested (Octree.impl.cuh:175-190).
 template <bool COUNT>
 __device__ __forceinline__ int lane_start(const Scene &S, LaneRay &L) {
-    L.inv = mkf3(__fdiv_rn(1.0f, L.d.x), __fdiv_rn(1.0f, L.d.y), __fdiv_rn(1.0f, L.d.z));
+    const f3 inv = mkf3(__fdiv_rn(1.0f, L.d.x), __fdiv_rn(1.0f, L.d.y), __fdiv_rn(1.0f, L.d.z));
+    if (COUNT) L.inv = inv;
     L.order = (L.d.z < 0 ? 1 : 0) + (L.d.y < 0 ? 2 : 0) + (L.d.x < 0 ? 4 : 0);
     L.sp = 0;
     L.cur = 0;
@@ -51,21 +64,46 @@ __device__ __forceinline__ int lane_start(const Scene &S, LaneRay &L) {
     if (S.root_child < 0) {
         L.r = S.root_leaf_first;
         L.r_end = S.root_leaf_first + S.root_leaf_count;
-        L.lx = S.root_lo[0]; L.ly = S.root_lo[1]; L.lz = S.root_lo[2];
-        L.hx = S.root_hi[0]; L.hy = S.root_hi[1]; L.hz = S.root_hi[2];
+        L.node = -1;
+        if (COUNT) {
+            L.lx = S.root_lo[0]; L.ly = S.root_lo[1]; L.lz = S.root_lo[2];
+            L.hx = S.root_hi[0]; L.hy = S.root_hi[1]; L.hz = S.root_hi[2];
+        }
         L.best = FLT_MAX;
-        L.bi = -1;
         L.kleaf = 7;  // no group scan to correct for a root leaf
         return kLeaf;
     }
     if (COUNT) L.nb++;
     const bool front = !COUNT || S.front_only != 0;
-    if (slab_hit(S.root_lo[0], S.root_lo[1], S.root_lo[2], S.root_hi[0], S.root_hi[1], S.root_hi[2], L.o, L.inv, front)) {
-        L.cur = ((uint32_t)S.root_child << group_shift<COUNT>()) |
-                test_group(front ? S.gbox : S.gbox_ref, S.root_child, L.order, L.o, L.inv, front);
-        if (COUNT) L.nb += 8;
+    if (slab_hit(S.root_lo[0], S.root_lo[1], S.root_lo[2], S.root_hi[0], S.root_hi[1], S.root_hi[2], L.o, inv, front)) {
+        if (COUNT) {
+            L.cur = ((uint32_t)S.root_child << kCountShift) |
+                    test_group(front ? S.gbox : S.gbox_ref, S.root_child, L.order, L.o, inv, front);
+            L.nb += 8;
+        } else {
+            // a frame whose one child left is the root's group: the first step tests it
+            L.k = ray_slopes(L.o, L.d, S.reach);
+            L.cur = never_hits(L.o, L.d) ? 0u : 1u;
+            L.links = ((uint32_t)S.root_child << 8) | (1u << L.order);
+        }
     }
     return kTrav;
+}
+
+// Whether the nearest hit of a leaf ends the ray (castInLeaf's acceptance): its point lies in the
+// leaf's box (or `anywhere`: an occluder), and the ray passes the exact slab test of that box, which
+// the conservative group tests on the way down stand in for.
+__device__ __forceinline__ bool leaf_accepts(const Scene &S, int node, f3 root_lo, f3 root_hi, f3 o, f3 d, f3 p, bool anywhere) {
+    f3 l = root_lo, h = root_hi;
+    if (node >= 0) {
+        float4 lo, hi;
+        ldg2(S.nodes + 2 * (size_t)node, lo, hi);
+        l = f3of(lo);
+        h = f3of(hi);
+        const f3 inv = mkf3(__fdiv_rn(1.0f, d.x), __fdiv_rn(1.0f, d.y), __fdiv_rn(1.0f, d.z));
+        if (!slab_hit(l.x, l.y, l.z, h.x, h.y, h.z, o, inv, true)) return false;
+    }
+    return anywhere || (p.x >= l.x && p.y >= l.y && p.z >= l.z && p.x <= h.x && p.y <= h.y && p.z <= h.z);
 }
 
 // Loads entry i of the source into the lane and starts its ray; kIdle when the source has nothing
@@ -88,6 +126,7 @@ struct WarpLeafSlots {
 // Source interface:
 //   bool next(int &begin, int &end)           warp-uniform; false when no work is left
 //   bool load(int i, f3 &o, f3 &d, int &ignore, int &job)   false: entry i needs no cast (done)
+//   int job(int i)                            the job of entry i
 //   const Scene &scene(int job)               the scene of a job (MULTI only)
 //   bool clip(int job)                        backface culling of a job (MULTI = false: job 0 for all)
 //   bool store(int i, const Hit &h, int nbox, int ntri)   true: ray i was rewritten (load() now
@@ -102,7 +141,7 @@ template <bool COUNT, bool MULTI, class Source>
 // steps_per_round: traversal steps a lane may take between two cooperative leaf rounds while it
 // stays in inner nodes; more means fewer per-round ballots and prefix sums, but lanes that reached a
 // leaf wait longer (measured: 2 pays on physical-tree scenes, whose leaves are small; 1 elsewhere).
-__device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, uint32_t *stack, WarpLeafSlots &ws,
+__device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, typename StackOf<COUNT>::type *stack, WarpLeafSlots &ws,
                                                  int steps_per_round = 1) {
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt_mask = (1u << lane) - 1u;
@@ -110,34 +149,42 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ui
     bool drained = false;
     int cur_i = -1;
     int mode = kIdle;
-    constexpr int GS = group_shift<COUNT>();
     const bool clip = src.clip(0);
     const bool front = !COUNT || S.front_only != 0;   // uniform: one scene, or one arena of a batch
     // group-test planes: refitted, except for counting on reference-padding scenes (their counts are
     // the reference's)
-    const float4 *G = front ? S.gbox : S.gbox_ref;
+    [[maybe_unused]] const float4 *G = front ? S.gbox : S.gbox_ref;
     LaneRay L;
     L.r = 0;
     L.r_end = 0;
     L.sp = 0;
     L.cur = 0;
     L.best = FLT_MAX;
-    L.bi = -1;
     for (;;) {
         // ---- refill idle lanes from the warp's chunk (warp-uniform control flow)
-        unsigned want = __ballot_sync(0xFFFFFFFFu, mode == kIdle);
+        bool start = false;
+        if (mode == kDone) {
+            Hit h;
+            h.tri = L.pos >= 0 ? __float_as_int(__ldg(S.leaf_tris + 3 * (size_t)L.pos).w) : -1;
+            h.t = L.best;
+            h.p = xadd(L.o, xmul(L.d, L.best));
+            start = src.store(cur_i, h, L.nb, L.nt);
+            mode = kIdle;
+        }
+        unsigned want = __ballot_sync(0xFFFFFFFFu, mode == kIdle && !start);
         if (want != 0u && !drained) {
             if (c_next >= c_end && !src.next(c_next, c_end)) drained = true;
             if (!drained) {
                 int avail = c_end - c_next;
                 int rank = __popc(want & lt_mask);
-                if (mode == kIdle && rank < avail) {
+                if (mode == kIdle && !start && rank < avail) {
                     cur_i = c_next + rank;
-                    mode = restart<COUNT, MULTI>(S, src, cur_i, L);
+                    start = true;
                 }
                 c_next += min(avail, __popc(want));
             }
         }
+        if (start) mode = restart<COUNT, MULTI>(S, src, cur_i, L);
         if (__ballot_sync(0xFFFFFFFFu, mode != kIdle) == 0u) {
             if (drained) break;
             continue;
@@ -146,18 +193,23 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ui
         for (int step = 0; step < steps_per_round; step++) {
         if (mode != kTrav) break;
         {
-            // ---- one traversal step: pop empty frames, then take one child
-            while ((L.cur & 0xFFu) == 0u && L.sp > 0) L.cur = stack[--L.sp];
-            uint32_t m = L.cur & 0xFFu;
+            // ---- one traversal step: pop an empty frame, then take one child
+            if constexpr (COUNT) {
+                while ((L.cur & 0xFFu) == 0u && L.sp > 0) L.cur = stack[--L.sp];
+            } else if ((L.cur & 0xFFu) == 0u && L.sp > 0) {   // frames are stacked with children left
+                const uint2 e = stack[--L.sp];
+                L.cur = e.x;
+                L.links = e.y;
+            }
+            const uint32_t m = L.cur & 0xFFu;
             if (m == 0u) {
-                Hit h;
-                h.tri = -1;
-                h.t = FLT_MAX;
-                mode = src.store(cur_i, h, L.nb, L.nt) ? restart<COUNT, MULTI>(S, src, cur_i, L) : kIdle;
-            } else {
+                L.pos = -1;
+                L.best = FLT_MAX;
+                mode = kDone;
+            } else if constexpr (COUNT) {
                 int k = __ffs(m) - 1;
                 L.cur &= ~(1u << k);
-                int node = (int)(L.cur >> GS) * 8 + (L.order ^ k);
+                int node = (int)(L.cur >> kCountShift) * 8 + (L.order ^ k);
                 float4 lo, hi;
                 ldg2(S.nodes + 2 * (size_t)node, lo, hi);
                 int w = __float_as_int(lo.w);
@@ -167,16 +219,37 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ui
                     L.lx = lo.x; L.ly = lo.y; L.lz = lo.z;
                     L.hx = hi.x; L.hy = hi.y; L.hz = hi.z;
                     L.best = FLT_MAX;
-                    L.bi = -1;
                     L.kleaf = k;
                     mode = kLeaf;
                 } else if (L.sp < kStack) {
-                    stack[L.sp++] = COUNT ? ((L.cur & ~(7u << 8)) | ((uint32_t)k << 8)) : L.cur;
-                    L.cur = ((uint32_t)(w >> 3) << GS) | test_group(G, w >> 3, L.order, L.o, L.inv, front);
-                    if (COUNT) L.nb += 8;
+                    stack[L.sp++] = (L.cur & ~(7u << 8)) | ((uint32_t)k << 8);
+                    L.cur = ((uint32_t)(w >> 3) << kCountShift) | test_group(G, w >> 3, L.order, L.o, L.inv, front);
+                    L.nb += 8;
                 } else {  // unreachable for depth <= 24: finish as a miss rather than overflow
                     L.cur = 0;
                     L.sp = 0;
+                }
+            } else {
+                const uint32_t c = (uint32_t)(__ffs(m) - 1) ^ (uint32_t)L.order;
+                L.cur &= L.cur - 1u;
+                const uint32_t g = L.cur >> 8;
+                if (((L.links >> c) & 1u) == 0u) {
+                    const int *first = reinterpret_cast<const int *>(S.groups + (size_t)g * kRecordF4) + 49 + c;
+                    L.r = __ldg(first);
+                    L.r_end = __ldg(first + 1);
+                    L.node = (int)(8u * g + c);
+                    L.best = FLT_MAX;
+                    mode = kLeaf;
+                } else {
+                    const uint32_t child = (L.links >> 8) + __popc(L.links & ((1u << c) - 1u));
+                    bool room = true;
+                    if ((L.cur & 0xFFu) != 0u) {
+                        room = L.sp < kStack;   // always for depth <= 24: finish as a miss rather than overflow
+                        if (room) stack[L.sp++] = make_uint2(L.cur, L.links);
+                    }
+                    L.cur = 0;
+                    if (room) L.cur = (child << 8) | record_mask(S.groups, child, L.order, L.k, L.links);
+                    else L.sp = 0;
                 }
             }
         }
@@ -252,8 +325,7 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ui
                     const float dist = __uint_as_float((unsigned)(k >> 32));
                     const int pos = (int)(k & 0xFFFFFFFFull);
                     L.best = dist;
-                    L.bi = __float_as_int(__ldg(S.leaf_tris + 3 * (size_t)pos).w);
-                    L.bp = xadd(L.o, xmul(L.d, dist));
+                    L.pos = pos;
                 }
             }
             __syncwarp();
@@ -261,20 +333,22 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ui
         if (mode == kLeaf && L.r >= L.r_end) {
             // occlusion sources end a ray at the first leaf holding a hit nearer than their limit, even
             // one whose point lies in a later leaf: that hit's own leaf would end the ray there anyway
-            const bool occluded = Source::kOccludeBelow > 0.0f && L.best < Source::kOccludeBelow;
-            if (L.best != FLT_MAX && (occluded || (L.bp.x >= L.lx && L.bp.y >= L.ly && L.bp.z >= L.lz && L.bp.x <= L.hx &&
-                                                   L.bp.y <= L.hy && L.bp.z <= L.hz))) {
-                if (COUNT) {
-                    L.nb -= 7 - L.kleaf;
-                    for (int s = 0; s < L.sp; s++) L.nb -= 7 - (int)((stack[s] >> 8) & 7u);
+            mode = kTrav;
+            if (L.best != FLT_MAX) {
+                const bool occluded = Source::kOccludeBelow > 0.0f && L.best < Source::kOccludeBelow;
+                const f3 p = xadd(L.o, xmul(L.d, L.best));
+                if constexpr (COUNT) {
+                    if (occluded || (p.x >= L.lx && p.y >= L.ly && p.z >= L.lz && p.x <= L.hx && p.y <= L.hy && p.z <= L.hz)) {
+                        L.nb -= 7 - L.kleaf;
+                        for (int s = 0; s < L.sp; s++) L.nb -= 7 - (int)((stack[s] >> 8) & 7u);
+                        mode = kDone;
+                    }
+                } else {
+                    const Scene &own = MULTI && L.node < 0 ? src.scene(src.job(cur_i)) : S;
+                    if (leaf_accepts(S, L.node, mkf3(own.root_lo[0], own.root_lo[1], own.root_lo[2]),
+                                     mkf3(own.root_hi[0], own.root_hi[1], own.root_hi[2]), L.o, L.d, p, occluded))
+                        mode = kDone;
                 }
-                Hit h;
-                h.tri = L.bi;
-                h.t = L.best;
-                h.p = L.bp;
-                mode = src.store(cur_i, h, L.nb, L.nt) ? restart<COUNT, MULTI>(S, src, cur_i, L) : kIdle;
-            } else {
-                mode = kTrav;
             }
         }
     }
