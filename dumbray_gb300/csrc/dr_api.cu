@@ -414,16 +414,6 @@ dr_status dr_scene_create(const float *xyz, const float *nrm, const int32_t *mat
         nodes[2 * i] = make_float4(T.node_lo[3 * i], T.node_lo[3 * i + 1], T.node_lo[3 * i + 2], wf);
         nodes[2 * i + 1] = make_float4(T.node_hi[3 * i], T.node_hi[3 * i + 1], T.node_hi[3 * i + 2], cf);
     }
-    std::vector<float4> leaf_tris(3 * T.leaf_refs.size());
-    for (size_t r = 0; r < T.leaf_refs.size(); r++) {
-        int id = T.leaf_refs[r];
-        const float *p = &sc->xyz[9 * (size_t)id];
-        float idf;
-        std::memcpy(&idf, &id, 4);
-        leaf_tris[3 * r] = make_float4(p[0], p[1], p[2], idf);
-        leaf_tris[3 * r + 1] = make_float4(p[3], p[4], p[5], 0.0f);
-        leaf_tris[3 * r + 2] = make_float4(p[6], p[7], p[8], 0.0f);
-    }
     std::vector<float4> tris(3 * (size_t)n), nrms(3 * (size_t)n);
     for (int64_t i = 0; i < n; i++) {
         const float *p = &sc->xyz[9 * i];
@@ -484,13 +474,22 @@ dr_status dr_scene_create(const float *xyz, const float *nrm, const int32_t *mat
     cudaError_t e = upload(&d_nodes, nodes.data(), nodes.size());
     if (e == cudaSuccess) { sc->allocs.push_back(d_nodes); e = upload(&d_gbox, (const float4 *)gbox.data(), gbox.size() / 4); }
     if (e == cudaSuccess) { sc->allocs.push_back(d_gbox); e = upload(&d_gbox_ref, (const float4 *)gbox_ref.data(), gbox_ref.size() / 4); }
-    if (e == cudaSuccess) { sc->allocs.push_back(d_gbox_ref); e = upload(&d_leaf, leaf_tris.data(), leaf_tris.size()); }
-    if (e == cudaSuccess) { sc->allocs.push_back(d_leaf); e = upload(&d_tris, tris.data(), tris.size()); }
+    if (e == cudaSuccess) { sc->allocs.push_back(d_gbox_ref); e = upload(&d_tris, tris.data(), tris.size()); }
     if (e == cudaSuccess) { sc->allocs.push_back(d_tris); e = upload(&d_nrms, nrms.data(), nrms.size()); }
     if (e == cudaSuccess) { sc->allocs.push_back(d_nrms); e = upload(&d_mat, sc->mat_id.data(), sc->mat_id.size()); }
     if (e == cudaSuccess) { sc->allocs.push_back(d_mat); e = upload(&d_mats, dm.data(), dm.size()); }
     if (e == cudaSuccess) { sc->allocs.push_back(d_mats); e = upload(&d_lights, dl.data(), dl.size()); }
     if (e == cudaSuccess) sc->allocs.push_back(d_lights);
+    const size_t n_refs = T.leaf_refs.size();
+    int *d_refs = nullptr;
+    if (e == cudaSuccess) e = upload(&d_refs, T.leaf_refs.data(), n_refs);
+    if (e == cudaSuccess && n_refs) e = cudaMalloc((void **)&d_leaf, sizeof(float4) * drd::kLeafTriF4 * n_refs);
+    if (e == cudaSuccess && n_refs) {
+        sc->allocs.push_back(d_leaf);
+        e = drk::launch_leaf_tris(d_leaf, d_refs, d_tris, (long long)n_refs, nullptr);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+    }
+    cudaFree(d_refs);
     float reach = 0.0f;
     for (int k = 0; k < 3; k++) reach = std::fmax(reach, std::fmax(std::fabs(T.root_lo[k]), std::fabs(T.root_hi[k])));
     const int64_t n_groups = T.node_count / 8;
@@ -505,7 +504,7 @@ dr_status dr_scene_create(const float *xyz, const float *nrm, const int32_t *mat
         return cuda_fail(e, "dr_scene_create: upload");
     }
     sc->node_f4 = (int64_t)nodes.size();
-    sc->leaf_f4 = (int64_t)leaf_tris.size();
+    sc->leaf_f4 = (int64_t)(drd::kLeafTriF4 * n_refs);
     drd::Scene &S = sc->dev;
     S.nodes = d_nodes;
     S.gbox = d_gbox;
@@ -1193,22 +1192,22 @@ static dr_status build_arena(dr_batch *b) {
         if ((sc->node_f4 / 2) % 8 != 0) return fail(DR_E_STATE, "dr_batch_create: octree nodes are not in groups of 8");
         uniq.push_back(sc);
         node_off.push_back(nodes / 2);
-        leaf_off.push_back(leaf / 3);
+        leaf_off.push_back(leaf / drd::kLeafTriF4);
         nodes += sc->node_f4;
         leaf += sc->leaf_f4;
     }
     b->arena_node_count = nodes / 2;
-    if (b->arena_node_count >= (int64_t(1) << 27) || leaf / 3 >= (int64_t(1) << 31))
+    if (b->arena_node_count >= (int64_t(1) << 27) || leaf / drd::kLeafTriF4 >= (int64_t(1) << 31))
         return fail(DR_E_CAPACITY, "dr_batch_create: the scenes' octrees exceed 2^27 nodes or 2^31 leaf references");
     cudaError_t e = cudaMalloc((void **)&b->arena_nodes, sizeof(float4) * (size_t)std::max<int64_t>(nodes, 2));
-    if (e == cudaSuccess) e = cudaMalloc((void **)&b->arena_leaf, sizeof(float4) * (size_t)std::max<int64_t>(leaf, 3));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&b->arena_leaf, sizeof(float4) * (size_t)std::max<int64_t>(leaf, 1));
     if (e == cudaSuccess) e = cudaMalloc((void **)&b->arena_gbox, sizeof(float4) * 12 * (size_t)std::max<int64_t>(nodes / 16, 1));
     if (e == cudaSuccess)
         e = cudaMalloc((void **)&b->arena_groups, sizeof(float4) * drd::kRecordF4 * (size_t)std::max<int64_t>(nodes / 16, 1));
     for (size_t k = 0; k < uniq.size() && e == cudaSuccess; k++) {
         const dr_scene *sc = uniq[k];
         if (sc->leaf_f4)
-            e = cudaMemcpy(b->arena_leaf + 3 * leaf_off[k], sc->dev.leaf_tris, sizeof(float4) * (size_t)sc->leaf_f4,
+            e = cudaMemcpy(b->arena_leaf + drd::kLeafTriF4 * leaf_off[k], sc->dev.leaf_tris, sizeof(float4) * (size_t)sc->leaf_f4,
                            cudaMemcpyDeviceToDevice);
         if (e == cudaSuccess && sc->node_f4)
             e = cudaMemcpy(b->arena_gbox + 12 * (node_off[k] / 8), sc->dev.gbox, sizeof(float4) * 12 * (size_t)(sc->node_f4 / 16),

@@ -6,8 +6,9 @@
 //              children of an inner node are 8 consecutive nodes, 8-aligned (one 256-byte group).
 //   groups     float4[16 * groups]     one 256-byte record per inner node: what a cast reads to test the
 //              8 children and to find the taken one (GroupRecord below)
-//   leaf_tris  float4[3 * refs]        leaf reference r = {a.xyz, w = triangle id}, {b.xyz}, {c.xyz}:
-//              the leaf's triangles duplicated in leaf order, so a leaf is one contiguous stream.
+//   leaf_tris  float4[4 * refs]        leaf reference r: the triangle's vertices and what of its test does
+//              not depend on the ray (LeafTri below), duplicated in leaf order, so a leaf is one
+//              contiguous stream.
 //   tris       float4[3 * n]           triangles by id (shading, light sampling)
 // The cast reproduces DumbRay's Octree::cast (Octree.impl.cuh:174-212) bit for bit: every
 // floating-point operation of the slab test, the triangle plane test and the edge-angle
@@ -130,55 +131,76 @@ __device__ __forceinline__ bool slab_hit(float lx, float ly, float lz, float hx,
     return mn != FLT_MAX;
 }
 
-// One edge condition of Triangle::containsVertex (Triangle.impl.h:292-302):
-//     rn(rn(X / rn(sqrt(P))) + S) >= rn(Y / rn(sqrt(Q)))
-// with X = e.px, P = px.px, Y = -(e.f), Q = f.f (all exactly rounded dot products).
-// Decided first with rsqrtf (documented max error 2 ulp): the fast left and right sides differ from
-// the exactly rounded ones by at most ~3 ulp each, so a difference D outside the margin
-// M = 2^-19 (|L| + |R| + S) (about 16 ulp) has the same sign as the exact difference; inside the
-// margin, or for inf/NaN operands, the exact IEEE expression is evaluated.  Results are therefore
-// bit-identical to the reference's host arithmetic while the common case avoids two IEEE divisions
-// and two IEEE square roots.
-__device__ __forceinline__ bool edge_ok(f3 e, f3 px, f3 f) {
-    const float S = 32 * kEps;
-    const float X = xdot(e, px), P = xdot(px, px), Y = -xdot(e, f), Q = xdot(f, f);
-    const float Lf = __fadd_rn(__fmul_rn(X, rsqrtf(P)), S);
-    const float Rf = __fmul_rn(Y, rsqrtf(Q));
-    const float D = __fsub_rn(Lf, Rf);
-    const float M = 1.9073486328125e-06f * (fabsf(Lf) + fabsf(Rf) + S);
-    if (D > M) return true;
-    if (D < -M) return false;
-    return __fadd_rn(__fdiv_rn(X, __fsqrt_rn(P)), S) >= __fdiv_rn(Y, __fsqrt_rn(Q));
+// One edge condition of Triangle::containsVertex (Triangle.impl.h:292-302), every operation exactly
+// rounded: rn(rn(X / rn(sqrt(P))) + S) >= rn(Y / rn(sqrt(Q))), X = e.px, P = px.px, Y = -(e.f), Q = f.f.
+// The right side depends on the triangle alone (edge_limit).
+constexpr float kEdgeSlack = 32 * kEps;
+__device__ __forceinline__ float edge_limit(f3 e, f3 f) { return __fdiv_rn(-xdot(e, f), __fsqrt_rn(xdot(f, f))); }
+__device__ __forceinline__ bool edge_ok(f3 e, f3 px, float limit) {
+    return __fadd_rn(__fdiv_rn(xdot(e, px), __fsqrt_rn(xdot(px, px))), kEdgeSlack) >= limit;
 }
 
-// Triangle::containsVertex (Triangle.impl.h:283-302)
-__device__ __forceinline__ bool contains_vertex(f3 a, f3 b, f3 c, f3 p) {
+// Triangle::containsVertex (Triangle.impl.h:283-302); `limit` = edge_limit at a, b, c.  Out of line:
+// reached by points on a vertex or within rounding of an edge angle only.
+static __device__ __noinline__ bool contains_vertex(f3 a, f3 b, f3 c, f3 p, float limit_a, float limit_b, float limit_c) {
     if (xeq(a, b) || xeq(b, c) || xeq(c, a)) return false;
     if (xeq(p, a) || xeq(p, b) || xeq(p, c)) return true;
-    f3 ab = xsub(b, a), bc = xsub(c, b), ca = xsub(a, c);
-    if (!edge_ok(ab, xsub(p, a), ca)) return false;
-    if (!edge_ok(bc, xsub(p, b), ab)) return false;
-    return edge_ok(ca, xsub(p, c), bc);
+    return edge_ok(xsub(b, a), xsub(p, a), limit_a) && edge_ok(xsub(c, b), xsub(p, b), limit_b) &&
+           edge_ok(xsub(a, c), xsub(p, c), limit_c);
 }
 
-// Triangle::cast (Triangle.impl.h:334-348), with the caller's strict-min and validator checks
-// (castInLeaf, Octree.impl.cuh:596-603) moved ahead of the containment test: a triangle whose
-// distance is not below `best`, or that is the ignored object, cannot change the leaf's result,
-// so skipping its containment test leaves every result unchanged.
-__device__ __forceinline__ bool tri_cast_better(f3 a, f3 b, f3 c, int id, f3 o, f3 d, bool clip, int ignore, float best,
-                                                float &dist, f3 &hp) {
-    f3 n = xcross(xsub(b, a), xsub(c, a));
-    float dp = xdot(xsub(a, o), n);
-    if (clip && (dp < -kEps)) return false;
-    float dirp = xdot(d, n);
-    if (__fmul_rn(dp, dirp) <= 0.0f) return false;
-    float distance = __fdiv_rn(dp, dirp);
-    if (!(distance < best) || id == ignore) return false;
-    f3 hv = xadd(o, xmul(d, distance));
-    if (!contains_vertex(a, b, c, hv)) return false;
-    dist = distance;
-    hp = hv;
-    return true;
+// An edge condition with rsqrtf (documented max error 2 ulp): the fast left side differs from the
+// exactly rounded one by at most ~3 ulp, so a difference D outside the margin
+// M = 2^-19 (|L| + |R| + S) (about 16 ulp) has the sign of the exact difference.  Returns D - M in
+// `in` (positive: certainly inside) and D + M in `out` (negative: certainly outside); both fail for
+// NaN and infinities, which leaves the decision to contains_vertex.
+__device__ __forceinline__ void edge_fast(f3 e, f3 px, float P, float limit, bool &in, bool &out) {
+    const float L = __fadd_rn(__fmul_rn(xdot(e, px), rsqrtf(P)), kEdgeSlack);
+    const float D = __fsub_rn(L, limit);
+    const float M = 1.9073486328125e-06f * (fabsf(L) + fabsf(limit) + kEdgeSlack);
+    in = in && D > M;
+    out = out || D < -M;
+}
+
+// Leaf reference (64 bytes): floats 0-8 the vertices a, b, c; 9-11 the plane normal (b - a) x (c - a);
+// 12-14 the right sides of the three edge conditions; 15 the triangle id.  The last seven are what a
+// test would otherwise compute again for every ray, with the same rounding.
+constexpr int kLeafTriF4 = 4;
+__device__ __forceinline__ int leaf_tri_id(const float4 *leaf_tris, int pos) {
+    return __float_as_int(__ldg(leaf_tris + (size_t)pos * kLeafTriF4 + 3).w);
+}
+__device__ __forceinline__ void ldg8(const void *p, float *v) {
+    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+        : "l"(p));
+}
+
+// Triangle::cast (Triangle.impl.h:334-348) of leaf reference `pos`, with the caller's validator check
+// (castInLeaf, Octree.impl.cuh:596-603) moved ahead of the containment test: the ignored triangle
+// cannot change the leaf's result.  The three edges are tested together: among the 32 tests of a
+// window some lane nearly always needs the last one.
+__device__ __forceinline__ bool tri_cast(const float4 *leaf_tris, int pos, f3 o, f3 d, bool clip, int ignore, float &dist) {
+    const float4 *q = leaf_tris + (size_t)pos * kLeafTriF4;
+    float u[8], w[8];
+    ldg8(q, u);
+    ldg8(q + 2, w);
+    const f3 a = mkf3(u[0], u[1], u[2]), b = mkf3(u[3], u[4], u[5]), c = mkf3(u[6], u[7], w[0]), n = mkf3(w[1], w[2], w[3]);
+    const float dp = xdot(xsub(a, o), n);
+    const float dirp = xdot(d, n);
+    if ((clip && dp < -kEps) || __fmul_rn(dp, dirp) <= 0.0f) return false;
+    dist = __fdiv_rn(dp, dirp);
+    if (!(dist < FLT_MAX) || __float_as_int(w[7]) == ignore) return false;
+    const f3 p = xadd(o, xmul(d, dist));
+    const f3 pa = xsub(p, a), pb = xsub(p, b), pc = xsub(p, c);
+    const float Pa = xdot(pa, pa), Pb = xdot(pb, pb), Pc = xdot(pc, pc);
+    bool in = fminf(fminf(Pa, Pb), Pc) > 0.0f, out = false;   // on a vertex: the exact test decides
+    const bool vertex = !in;
+    edge_fast(xsub(b, a), pa, Pa, w[4], in, out);
+    edge_fast(xsub(c, b), pb, Pb, w[5], in, out);
+    edge_fast(xsub(a, c), pc, Pc, w[6], in, out);
+    if (in) return true;
+    if (out && !vertex) return false;
+    return contains_vertex(a, b, c, p, w[4], w[5], w[6]);
 }
 
 struct Hit {
@@ -304,12 +326,6 @@ __device__ __forceinline__ RaySlopes ray_slopes(f3 o, f3 d, float reach) {
 __device__ __forceinline__ bool never_hits(f3 o, f3 d) {
     const float z = (o.x - o.x) + (o.y - o.y) + (o.z - o.z) + (d.x - d.x) + (d.y - d.y) + (d.z - d.z);
     return z != 0.0f || z != z || (d.x == 0.0f && d.y == 0.0f && d.z == 0.0f);
-}
-
-__device__ __forceinline__ void ldg8(const char *p, float *v) {
-    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-        : "l"(p));
 }
 
 // Children of group `g` that the ray may enter, bit k = child (order ^ k), and the group's word 48.

@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(128) k_cast(Scene S, const float *__restrict__
                                               const int *__restrict__ ignore, int n, int clip, int *__restrict__ hit_tri,
                                               float *__restrict__ hit_t, int *__restrict__ nbox, int *__restrict__ ntri) {
     typename StackOf<COUNT>::type stack[kStack];
-    __shared__ WarpLeafSlots slots[4];
+    __shared__ WarpSlots slots[4];
     BatchSource src{o, d, ignore, hit_tri, COUNT ? nbox : nullptr, COUNT ? ntri : nullptr, hit_t, n, false, clip != 0, &S};
     trace_persistent<COUNT, false>(S, src, stack, slots[threadIdx.x >> 5]);
 }
@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(TT, TB) k_trace(WaveArgs A, int b) {
     Ctrl *C = A.ctrl;
     const int n = *((volatile int *)&C->ray_count[b]);
     typename StackOf<COUNT>::type stack[kStack];
-    __shared__ WarpLeafSlots slots[TT / 32];
+    __shared__ WarpSlots slots[TT / 32];
     TraceSource<MULTI> src{&A, A.q[b & 1], A.hits, &C->fetch_trace[b], n, chunk_for(n), 0, 0, 0};
     trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], A.inl.S.front_only ? kPhysStepsPerRound : 1);
     if (COUNT) count_add64(A.counters, src.rays, src.nb, src.nt);
@@ -692,7 +692,7 @@ __global__ void __launch_bounds__(kTraceThreads, kShadowRefBlocksPerSM) k_shadow
     const int n = *((volatile int *)&C->shadow_count[b]);
     if (n == 0) return;
     typename StackOf<COUNT>::type stack[kStack];
-    __shared__ WarpLeafSlots slots[kTraceThreads / 32];
+    __shared__ WarpSlots slots[kTraceThreads / 32];
     RefPhotonSource<MULTI> src{&A, A.sq, &C->fetch_shadow[b], &C->carry_count, blocked_list(A, b), &C->blocked_count[b], n,
                                chunk_for(n), 0, 0, 0};
     trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5]);
@@ -708,7 +708,7 @@ __global__ void __launch_bounds__(kTraceThreads, kPhotonChainBlocksPerSM) k_phot
     const int n = carry ? min(*((volatile int *)&C->carry_count), A.carry_cap) : *((volatile int *)&C->blocked_count[b]);
     if (n == 0) return;
     typename StackOf<COUNT>::type stack[kStack];
-    __shared__ WarpLeafSlots slots[kTraceThreads / 32];
+    __shared__ WarpSlots slots[kTraceThreads / 32];
     RefPhotonChainSource<MULTI> src{&A, carry ? A.cq : A.sq, carry ? nullptr : blocked_list(A, b),
                                     carry ? &C->fetch_carry : &C->fetch_chain[b], n, chunk_for(n), 0, 0, 0};
     trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5]);
@@ -992,7 +992,7 @@ __global__ void __launch_bounds__(TT, TB) k_shadow_phys(WaveArgs A, int b) {
     Ctrl *C = A.ctrl;
     const int n = *((volatile int *)&C->shadow_count[b]);
     typename StackOf<COUNT>::type stack[kStack];
-    __shared__ WarpLeafSlots slots[TT / 32];
+    __shared__ WarpSlots slots[TT / 32];
     ShadowPhysSource<MULTI, ADJ> src{&A, A.sq, A.accum, &C->fetch_shadow[b], n, chunk_for(n), 0, 0, 0};
     trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], A.inl.S.front_only ? kPhysStepsPerRound : 1);
     if (COUNT) count_add64(A.counters + 3, src.rays, src.nb, src.nt);
@@ -1032,6 +1032,21 @@ __global__ void k_resolve(WaveArgs A, int total_slots) {
         float4 old = fb[at];
         fb[at] = make_float4((c.x * blend) + (old.x * (1.0f - blend)), (c.y * blend) + (old.y * (1.0f - blend)),
                              (c.z * blend) + (old.z * (1.0f - blend)), (c.w * blend) + (old.w * (1.0f - blend)));
+    }
+}
+
+// Leaf references (kLeafTriF4 layout) from the triangles: one thread per reference.
+__global__ void k_leaf_tris(float4 *dst, const int *refs, const float4 *tris, long long n_refs) {
+    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < n_refs; r += (long long)gridDim.x * blockDim.x) {
+        const int id = refs[r];
+        const TriV t = load_tri(tris, id);
+        const f3 ab = xsub(t.b, t.a), bc = xsub(t.c, t.b), ca = xsub(t.a, t.c);
+        const f3 n = xcross(ab, xsub(t.c, t.a));
+        float4 *q = dst + r * kLeafTriF4;
+        q[0] = make_float4(t.a.x, t.a.y, t.a.z, t.b.x);
+        q[1] = make_float4(t.b.y, t.b.z, t.c.x, t.c.y);
+        q[2] = make_float4(t.c.z, n.x, n.y, n.z);
+        q[3] = make_float4(edge_limit(ab, ca), edge_limit(bc, ab), edge_limit(ca, bc), __int_as_float(id));
     }
 }
 
@@ -1329,6 +1344,13 @@ cudaError_t launch_rebase_nodes(float4 *dst, const float4 *src, long long n_node
     if (n_nodes <= 0) return cudaSuccess;
     const int grid = (int)std::min<long long>((n_nodes + 255) / 256, (long long)sm_count() * 8);
     drd::k_rebase_nodes<<<grid, 256, 0, stream>>>(dst, src, n_nodes, group_off, leaf_off);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_leaf_tris(float4 *dst, const int *refs, const float4 *tris, long long n_refs, cudaStream_t stream) {
+    if (n_refs <= 0) return cudaSuccess;
+    const int grid = (int)std::min<long long>((n_refs + 255) / 256, (long long)sm_count() * 32);
+    drd::k_leaf_tris<<<grid, 256, 0, stream>>>(dst, refs, tris, n_refs);
     return cudaGetLastError();
 }
 

@@ -106,6 +106,8 @@ cudaError_t launch_wave(const WaveDesc &W, cudaStream_t stream, long long *launc
 // index 8 * group_off), adding the offsets to child node and first-leaf-reference indices.
 cudaError_t launch_rebase_nodes(float4 *dst, const float4 *src, long long n_nodes, int group_off, int leaf_off,
                                 cudaStream_t stream);
+// Leaf references (drd::kLeafTriF4 float4 each) from the triangle ids in leaf order.
+cudaError_t launch_leaf_tris(float4 *dst, const int *refs, const float4 *tris, long long n_refs, cudaStream_t stream);
 // Group records (drd::kRecordF4 float4 each) of a scene from its nodes and refitted planes, boxes
 // widened by `pad`; and their copy into a batch arena at group `group_off`, leaf reference `leaf_off`.
 cudaError_t launch_group_records(float4 *dst, const float4 *nodes, const float4 *gbox, long long n_groups, float pad,

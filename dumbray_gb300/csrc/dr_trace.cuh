@@ -1,20 +1,30 @@
 // dr_trace.cuh - persistent, warp-refilled octree traversal for ray batches.
 //
 // Each lane traces one ray at a time with exactly the visit order and leaf semantics of
-// Octree::cast (Octree.impl.cuh:174-212, castInLeaf :584-612), so results are identical to
-// cast_closest().  What changes is the scheduling across the 32 lanes of a warp:
-//   * one unit of work per lane per loop iteration: either one traversal step (stack pops plus at
-//     most one 8-child group test, or entering a leaf) or one triangle test.  A lane never waits
-//     for another lane's whole leaf or whole descent; per-ray costs range over three orders of
-//     magnitude on displaced meshes (p99 ~1,700 triangle tests against a mean of ~120);
+// Octree::cast (Octree.impl.cuh:174-212, castInLeaf :584-612), so results are identical to a
+// one-ray-at-a-time cast.  What changes is the scheduling across the 32 lanes of a warp:
+//   * one unit of work per lane per loop iteration: a few traversal steps (at most one 8-child group
+//     test each, or entering a leaf), then one leaf round.  A lane never waits for another lane's
+//     whole descent; per-ray costs range over three orders of magnitude on displaced meshes (p99
+//     ~1,700 triangle tests against a mean of ~120);
 //   * leaf work is shared by the whole warp: the pending (ray, triangle) tests of all lanes that hold
-//     a leaf are numbered with a warp prefix sum and handed out 64 per round, two per lane; the
-//     tester reads the owner's ray through shuffles and posts (distance, list position) to the
-//     owner's slot with a 64-bit atomicMin, so the owner keeps the smallest distance and, among
-//     equal distances, the earliest triangle in list order - exactly castInLeaf's strict-min scan;
+//     a leaf are numbered by ballots and handed out 32 at a time, one per lane, until none is left;
+//     the tester reads the owner's ray from the warp's shared slots and posts (distance, list
+//     position) to the owner's key with a 64-bit atomicMin, so the owner keeps the smallest distance
+//     and, among equal distances, the earliest triangle in list order - exactly castInLeaf's
+//     strict-min scan;
 //   * a lane whose ray is finished takes the next ray of the warp's current chunk at once.  Chunks
 //     are handed out by the caller's Source (an atomic counter for queues whose size is only known
 //     on the device, a fixed range for plain batches).
+// A ray's origin, direction and ignored triangle live in shared memory only: the testers need them
+// from another lane and its own lane rarely does, so they cost no registers during the descent.
+//
+// The kernels are bound by instruction issue and by each iteration's latency, so a round is kept short:
+// independent ballots number the tests instead of a chain of five shuffles, a set bit per owner and one
+// shared read find a test's owner instead of a five-step search, a window of 32 is skipped when empty.
+// Against 64 tests a round with prefix sum, search, ten shuffles and the triangle's constants computed
+// per test (same call): 1080p primary casts on the reference tree 2.57 -> 1.59 ms, room 13.2 -> 9.5 ms,
+// 1080p photon render 63.5 -> 44.2 ms, path trace 44.2 -> 38.5 ms, gradients 87.5 -> 74.8 ms.
 #pragma once
 #include "dr_device.cuh"
 
@@ -24,17 +34,24 @@ constexpr int kChunk = 256;
 
 enum : int { kIdle = 0, kTrav = 1, kLeaf = 2, kDone = 3 };
 
+// A warp's shared slots, one per lane.
+struct WarpSlots {
+    float4 o[32];                    // origin, ignored triangle
+    float4 d[32];                    // direction
+    unsigned long long key[32];      // nearest hit of the current leaf: distance bits << 32 | list position
+    int2 task[32];                   // round's k-th owner: its lane, its first reference - its first task
+};
+constexpr unsigned long long kNoHit = ~0ull;
+
 struct LaneRay {
-    f3 o, d, inv;                    // inv: counting traversals
+    f3 o, inv;                       // counting traversals
     RaySlopes k;                     // every other traversal
-    int order, ignore;
+    int order;
     uint32_t cur, links;             // group << shift | remaining hit mask; the group's word 48
     int sp;
     int r, r_end;
     int node;                        // leaf node being tested, -1 = the root is the leaf
     float lx, ly, lz, hx, hy, hz;    // its box (counting traversals)
-    float best;
-    int pos;                         // list position of the nearest triangle so far
     int kleaf;
     int nb, nt;
 };
@@ -52,15 +69,18 @@ struct StackOf<true> {
 
 // Starts a ray: root leaf, root miss, or the root's children tested (Octree.impl.cuh:175-190).
 template <bool COUNT>
-__device__ __forceinline__ int lane_start(const Scene &S, LaneRay &L) {
-    const f3 inv = mkf3(__fdiv_rn(1.0f, L.d.x), __fdiv_rn(1.0f, L.d.y), __fdiv_rn(1.0f, L.d.z));
-    if (COUNT) L.inv = inv;
-    L.order = (L.d.z < 0 ? 1 : 0) + (L.d.y < 0 ? 2 : 0) + (L.d.x < 0 ? 4 : 0);
+__device__ __forceinline__ int lane_start(const Scene &S, LaneRay &L, f3 o, f3 d) {
+    const f3 inv = mkf3(__fdiv_rn(1.0f, d.x), __fdiv_rn(1.0f, d.y), __fdiv_rn(1.0f, d.z));
+    L.order = (d.z < 0 ? 1 : 0) + (d.y < 0 ? 2 : 0) + (d.x < 0 ? 4 : 0);
     L.sp = 0;
     L.cur = 0;
-    L.nb = 0;
-    L.nt = 0;
-    L.kleaf = 0;
+    if (COUNT) {
+        L.o = o;
+        L.inv = inv;
+        L.nb = 0;
+        L.nt = 0;
+        L.kleaf = 0;
+    }
     if (S.root_child < 0) {
         L.r = S.root_leaf_first;
         L.r_end = S.root_leaf_first + S.root_leaf_count;
@@ -68,22 +88,21 @@ __device__ __forceinline__ int lane_start(const Scene &S, LaneRay &L) {
         if (COUNT) {
             L.lx = S.root_lo[0]; L.ly = S.root_lo[1]; L.lz = S.root_lo[2];
             L.hx = S.root_hi[0]; L.hy = S.root_hi[1]; L.hz = S.root_hi[2];
+            L.kleaf = 7;  // no group scan to correct for a root leaf
         }
-        L.best = FLT_MAX;
-        L.kleaf = 7;  // no group scan to correct for a root leaf
         return kLeaf;
     }
     if (COUNT) L.nb++;
     const bool front = !COUNT || S.front_only != 0;
-    if (slab_hit(S.root_lo[0], S.root_lo[1], S.root_lo[2], S.root_hi[0], S.root_hi[1], S.root_hi[2], L.o, inv, front)) {
+    if (slab_hit(S.root_lo[0], S.root_lo[1], S.root_lo[2], S.root_hi[0], S.root_hi[1], S.root_hi[2], o, inv, front)) {
         if (COUNT) {
             L.cur = ((uint32_t)S.root_child << kCountShift) |
-                    test_group(front ? S.gbox : S.gbox_ref, S.root_child, L.order, L.o, inv, front);
+                    test_group(front ? S.gbox : S.gbox_ref, S.root_child, L.order, o, inv, front);
             L.nb += 8;
         } else {
             // a frame whose one child left is the root's group: the first step tests it
-            L.k = ray_slopes(L.o, L.d, S.reach);
-            L.cur = never_hits(L.o, L.d) ? 0u : 1u;
+            L.k = ray_slopes(o, d, S.reach);
+            L.cur = never_hits(o, d) ? 0u : 1u;
             L.links = ((uint32_t)S.root_child << 8) | (1u << L.order);
         }
     }
@@ -110,18 +129,15 @@ __device__ __forceinline__ bool leaf_accepts(const Scene &S, int node, f3 root_l
 // to trace for it.  Also serves a ray the source rewrote in place (a photon continuing past a
 // blocker): the lane starts it at once, without going back to the warp's chunk.
 template <bool COUNT, bool MULTI, class Source>
-__device__ __forceinline__ int restart(const Scene &S, Source &src, int i, LaneRay &L) {
+__device__ __forceinline__ int restart(const Scene &S, Source &src, int i, LaneRay &L, WarpSlots &ws, unsigned lane) {
     int ign, job;
-    if (!src.load(i, L.o, L.d, ign, job)) return kIdle;
-    L.ignore = ign;
-    return lane_start<COUNT>(MULTI ? src.scene(job) : S, L);
+    f3 o, d;
+    if (!src.load(i, o, d, ign, job)) return kIdle;
+    ws.o[lane] = make_float4(o.x, o.y, o.z, __int_as_float(ign));
+    ws.d[lane] = make_float4(d.x, d.y, d.z, 0.0f);
+    ws.key[lane] = kNoHit;
+    return lane_start<COUNT>(MULTI ? src.scene(job) : S, L, o, d);
 }
-
-// Per-warp shared scratch of the cooperative leaf rounds.
-struct WarpLeafSlots {
-    unsigned long long key[32];
-    int incl[32];
-};
 
 // Source interface:
 //   bool next(int &begin, int &end)           warp-uniform; false when no work is left
@@ -137,12 +153,18 @@ struct WarpLeafSlots {
 // warp; their trees live in one batch arena (S.nodes / S.leaf_tris are the arena's), so a lane only
 // takes its scene's root (bounds, child group or root leaf) when it starts a ray.  Backface culling
 // is uniform over a wave in both cases.
+// Tests one lane may bring to a round, a bound on the ballots that number them; larger leaves (the
+// unsplittable ones) take several rounds.
+constexpr int kRoundBits = 5;
+constexpr int kRoundCap = (1 << kRoundBits) - 1;
+
+// steps_per_round: traversal steps a lane may take between two leaf rounds while it stays in inner
+// nodes; more means fewer rounds, but lanes that reached a leaf wait longer (measured: 2 pays on
+// physical-tree scenes, whose leaves are small; 1 elsewhere).
 template <bool COUNT, bool MULTI, class Source>
-// steps_per_round: traversal steps a lane may take between two cooperative leaf rounds while it
-// stays in inner nodes; more means fewer per-round ballots and prefix sums, but lanes that reached a
-// leaf wait longer (measured: 2 pays on physical-tree scenes, whose leaves are small; 1 elsewhere).
-__device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, typename StackOf<COUNT>::type *stack, WarpLeafSlots &ws,
+__device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, typename StackOf<COUNT>::type *stack, WarpSlots &ws,
                                                  int steps_per_round = 1) {
+    constexpr unsigned kAll = 0xFFFFFFFFu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt_mask = (1u << lane) - 1u;
     int c_next = 0, c_end = 0;
@@ -151,32 +173,38 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ty
     int mode = kIdle;
     const bool clip = src.clip(0);
     const bool front = !COUNT || S.front_only != 0;   // uniform: one scene, or one arena of a batch
-    // group-test planes: refitted, except for counting on reference-padding scenes (their counts are
-    // the reference's)
+    // group-test planes of a counting traversal: the reference's boxes on reference-padding scenes
+    // (their counts are the reference's), the refitted ones elsewhere
     [[maybe_unused]] const float4 *G = front ? S.gbox : S.gbox_ref;
     LaneRay L;
     L.r = 0;
     L.r_end = 0;
     L.sp = 0;
     L.cur = 0;
-    L.best = FLT_MAX;
+    L.nb = 0;
+    L.nt = 0;
     for (;;) {
-        // ---- refill idle lanes from the warp's chunk (warp-uniform control flow)
+        // ---- finished rays, then refill of idle lanes from the warp's chunk (warp-uniform control flow)
         bool start = false;
         if (mode == kDone) {
+            const unsigned long long key = ws.key[lane];
             Hit h;
-            h.tri = L.pos >= 0 ? __float_as_int(__ldg(S.leaf_tris + 3 * (size_t)L.pos).w) : -1;
-            h.t = L.best;
-            h.p = xadd(L.o, xmul(L.d, L.best));
+            h.tri = -1;
+            h.t = FLT_MAX;
+            if (key != kNoHit) {
+                h.tri = leaf_tri_id(S.leaf_tris, (int)(key & 0xFFFFFFFFull));
+                h.t = __uint_as_float((unsigned)(key >> 32));
+                h.p = xadd(f3of(ws.o[lane]), xmul(f3of(ws.d[lane]), h.t));
+            }
             start = src.store(cur_i, h, L.nb, L.nt);
             mode = kIdle;
         }
-        unsigned want = __ballot_sync(0xFFFFFFFFu, mode == kIdle && !start);
+        const unsigned want = __ballot_sync(kAll, mode == kIdle && !start);
         if (want != 0u && !drained) {
             if (c_next >= c_end && !src.next(c_next, c_end)) drained = true;
             if (!drained) {
-                int avail = c_end - c_next;
-                int rank = __popc(want & lt_mask);
+                const int avail = c_end - c_next;
+                const int rank = __popc(want & lt_mask);
                 if (mode == kIdle && !start && rank < avail) {
                     cur_i = c_next + rank;
                     start = true;
@@ -184,15 +212,14 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ty
                 c_next += min(avail, __popc(want));
             }
         }
-        if (start) mode = restart<COUNT, MULTI>(S, src, cur_i, L);
-        if (__ballot_sync(0xFFFFFFFFu, mode != kIdle) == 0u) {
+        if (start) mode = restart<COUNT, MULTI>(S, src, cur_i, L, ws, lane);
+        if (__ballot_sync(kAll, mode != kIdle) == 0u) {
             if (drained) break;
             continue;
         }
 #pragma unroll 1
         for (int step = 0; step < steps_per_round; step++) {
-        if (mode != kTrav) break;
-        {
+            if (mode != kTrav) break;
             // ---- one traversal step: pop an empty frame, then take one child
             if constexpr (COUNT) {
                 while ((L.cur & 0xFFu) == 0u && L.sp > 0) L.cur = stack[--L.sp];
@@ -203,9 +230,7 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ty
             }
             const uint32_t m = L.cur & 0xFFu;
             if (m == 0u) {
-                L.pos = -1;
-                L.best = FLT_MAX;
-                mode = kDone;
+                mode = kDone;   // a miss: the key holds no hit
             } else if constexpr (COUNT) {
                 int k = __ffs(m) - 1;
                 L.cur &= ~(1u << k);
@@ -218,7 +243,6 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ty
                     L.r_end = ~w + __float_as_int(hi.w);
                     L.lx = lo.x; L.ly = lo.y; L.lz = lo.z;
                     L.hx = hi.x; L.hy = hi.y; L.hz = hi.z;
-                    L.best = FLT_MAX;
                     L.kleaf = k;
                     mode = kLeaf;
                 } else if (L.sp < kStack) {
@@ -238,7 +262,6 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ty
                     L.r = __ldg(first);
                     L.r_end = __ldg(first + 1);
                     L.node = (int)(8u * g + c);
-                    L.best = FLT_MAX;
                     mode = kLeaf;
                 } else {
                     const uint32_t child = (L.links >> 8) + __popc(L.links & ((1u << c) - 1u));
@@ -253,90 +276,48 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ty
                 }
             }
         }
-        }
-        // ---- one cooperative round of leaf triangle tests (castInLeaf)
-        int pending = (mode == kLeaf) ? (L.r_end - L.r) : 0;
-        int incl = pending;
+        // ---- one leaf round (castInLeaf): up to kRoundCap tests of every lane that holds a leaf
+        const unsigned owners = __ballot_sync(kAll, mode == kLeaf && L.r < L.r_end);
+        if (owners != 0u) {
+            const bool mine = (owners >> lane) & 1u;
+            const int count = mine ? min(L.r_end - L.r, kRoundCap) : 0;
+            int before = 0, total = 0;   // tests of the lanes below; of all
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            int v = __shfl_up_sync(0xFFFFFFFFu, incl, off);
-            if ((int)lane >= off) incl += v;
-        }
-        const int total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-        if (total > 0) {
-            ws.incl[lane] = incl;
-            ws.key[lane] = ~0ull;
+            for (int j = 0; j < kRoundBits; j++) {
+                const unsigned b = __ballot_sync(kAll, (count >> j) & 1);
+                before += __popc(b & lt_mask) << j;
+                total += __popc(b) << j;
+            }
+            if (mine) ws.task[__popc(owners & lt_mask)] = make_int2((int)lane, L.r - before);
             __syncwarp();
-            // tasks `lane` and `lane + 32` of this round; task t belongs to the first lane whose
-            // inclusive count exceeds t.  Both triangles are loaded before either is tested.
-            const int t0 = (int)lane, t1 = (int)lane + 32;
-            int own0 = (int)lane, own1 = (int)lane;
-            if (t0 < total) {
-                own0 = 0;
-#pragma unroll
-                for (int step = 16; step > 0; step >>= 1)
-                    if (ws.incl[own0 + step - 1] <= t0) own0 += step;
-            }
-            if (t1 < total) {
-                own1 = 0;
-#pragma unroll
-                for (int step = 16; step > 0; step >>= 1)
-                    if (ws.incl[own1 + step - 1] <= t1) own1 += step;
-            }
-            const int excl0 = ws.incl[own0] - __shfl_sync(0xFFFFFFFFu, pending, own0);
-            const int excl1 = ws.incl[own1] - __shfl_sync(0xFFFFFFFFu, pending, own1);
-            const int r0 = __shfl_sync(0xFFFFFFFFu, L.r, own0), r1 = __shfl_sync(0xFFFFFFFFu, L.r, own1);
-            const int pos0 = r0 + (t0 - excl0), pos1 = r1 + (t1 - excl1);
-            float4 A0, B0, C0, A1, B1, C1;
-            if (t0 < total) {
-                const float4 *lt = S.leaf_tris + 3 * (size_t)pos0;
-                A0 = __ldg(lt); B0 = __ldg(lt + 1); C0 = __ldg(lt + 2);
-            }
-            if (t1 < total) {
-                const float4 *lt = S.leaf_tris + 3 * (size_t)pos1;
-                A1 = __ldg(lt); B1 = __ldg(lt + 1); C1 = __ldg(lt + 2);
-            }
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                const int own = q ? own1 : own0;
-                const float ox = __shfl_sync(0xFFFFFFFFu, L.o.x, own), oy = __shfl_sync(0xFFFFFFFFu, L.o.y, own),
-                            oz = __shfl_sync(0xFFFFFFFFu, L.o.z, own);
-                const float dx = __shfl_sync(0xFFFFFFFFu, L.d.x, own), dy = __shfl_sync(0xFFFFFFFFu, L.d.y, own),
-                            dz = __shfl_sync(0xFFFFFFFFu, L.d.z, own);
-                const int ign = __shfl_sync(0xFFFFFFFFu, L.ignore, own);
-                const float obest = __shfl_sync(0xFFFFFFFFu, L.best, own);
-                if ((q ? t1 : t0) < total) {
-                    const float4 A = q ? A1 : A0, B = q ? B1 : B0, C = q ? C1 : C0;
+            int owned = 0;   // owners whose tests began in an earlier window
+            for (int base = 0; base < total; base += 32) {
+                const int at = before - base;
+                const unsigned begins = __reduce_or_sync(kAll, mine && at >= 0 && at < 32 ? 1u << at : 0u);
+                const int t = base + (int)lane;
+                if (t < total) {
+                    const int2 task = ws.task[owned + __popc(begins & (lt_mask << 1 | 1u)) - 1];
+                    const int pos = task.y + t;
+                    const float4 o = ws.o[task.x], d = ws.d[task.x];
                     float dist;
-                    f3 hp;
-                    if (tri_cast_better(f3of(A), f3of(B), f3of(C), __float_as_int(A.w), mkf3(ox, oy, oz), mkf3(dx, dy, dz),
-                                        clip, ign, obest, dist, hp))
-                        atomicMin(&ws.key[own], ((unsigned long long)__float_as_uint(dist) << 32) | (unsigned)(q ? pos1 : pos0));
+                    if (tri_cast(S.leaf_tris, pos, f3of(o), f3of(d), clip, __float_as_int(o.w), dist))
+                        atomicMin(&ws.key[task.x], ((unsigned long long)__float_as_uint(dist) << 32) | (unsigned)pos);
                 }
+                owned += __popc(begins);
             }
             __syncwarp();
-            if (mode == kLeaf) {
-                const int excl = incl - pending;
-                const int done = max(0, min(pending, 64 - excl));
-                if (COUNT) L.nt += done;
-                L.r += done;
-                const unsigned long long k = ws.key[lane];
-                if (k != ~0ull) {
-                    const float dist = __uint_as_float((unsigned)(k >> 32));
-                    const int pos = (int)(k & 0xFFFFFFFFull);
-                    L.best = dist;
-                    L.pos = pos;
-                }
-            }
-            __syncwarp();
+            if (COUNT) L.nt += count;
+            L.r += count;
         }
         if (mode == kLeaf && L.r >= L.r_end) {
             // occlusion sources end a ray at the first leaf holding a hit nearer than their limit, even
             // one whose point lies in a later leaf: that hit's own leaf would end the ray there anyway
             mode = kTrav;
-            if (L.best != FLT_MAX) {
-                const bool occluded = Source::kOccludeBelow > 0.0f && L.best < Source::kOccludeBelow;
-                const f3 p = xadd(L.o, xmul(L.d, L.best));
+            const unsigned long long key = ws.key[lane];
+            if (key != kNoHit) {
+                const float t = __uint_as_float((unsigned)(key >> 32));
+                const bool occluded = Source::kOccludeBelow > 0.0f && t < Source::kOccludeBelow;
+                const f3 o = f3of(ws.o[lane]), d = f3of(ws.d[lane]), p = xadd(o, xmul(d, t));
                 if constexpr (COUNT) {
                     if (occluded || (p.x >= L.lx && p.y >= L.ly && p.z >= L.lz && p.x <= L.hx && p.y <= L.hy && p.z <= L.hz)) {
                         L.nb -= 7 - L.kleaf;
@@ -346,9 +327,10 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ty
                 } else {
                     const Scene &own = MULTI && L.node < 0 ? src.scene(src.job(cur_i)) : S;
                     if (leaf_accepts(S, L.node, mkf3(own.root_lo[0], own.root_lo[1], own.root_lo[2]),
-                                     mkf3(own.root_hi[0], own.root_hi[1], own.root_hi[2]), L.o, L.d, p, occluded))
+                                     mkf3(own.root_hi[0], own.root_hi[1], own.root_hi[2]), o, d, p, occluded))
                         mode = kDone;
                 }
+                if (mode != kDone) ws.key[lane] = kNoHit;
             }
         }
     }
