@@ -916,8 +916,8 @@ def run_batched(dr, torch, dev, a):
                                              else "inf": v for k, v in sorted(best_split.items())},
                      "leaf_probe_ms": {str(k): v for k, v in split_table.items()},
                      "wave": best_wave, "wave_probe_ms": {str(k): v for k, v in wave_table.items()},
-                     "block_shape": ["256x3", "128x6"][best_shape],
-                     "block_shape_probe_ms": {["256x3", "128x6"][k]: v for k, v in shape_table.items()}},
+                     "block_shape": ["256x4", "128x8"][best_shape],
+                     "block_shape_probe_ms": {["256x4", "128x8"][k]: v for k, v in shape_table.items()}},
         "job_mean_max_rel_diff_batched_vs_plain": float(rel.max()),
         "by_size_class": classes,
         "accuracy_vs_fp64_oracle": dict(acc, sample="4 jobs (the cheapest for the oracle of each resolution), "

@@ -664,7 +664,7 @@ class Renderer:
         check(lib().dr_renderer_set_lanes(self._h, int(lanes)))
 
     def set_block_shape(self, shape: int):
-        """Traversal block shape (dr_renderer_set_block_shape): 0 = 256 x 3, 1 = 128 x 6 per SM."""
+        """Traversal block shape (dr_renderer_set_block_shape): 0 = 256 x 4, 1 = 128 x 8 per SM."""
         check(lib().dr_renderer_set_block_shape(self._h, int(shape)))
 
     @property

@@ -8,7 +8,7 @@ Picks, by timing short renders on the GPU:
     Larger leaves trade child-box tests for triangle tests, which the cooperative warp-wide leaf
     rounds run well, so the best value depends on the triangle density of the scene.
   * the wave size (paths in flight per wave = queue capacity of the renderer) of a batch;
-  * the block shape of the traversal kernels (256 threads x 3 blocks or 128 x 6 per SM).
+  * the block shape of the traversal kernels (256 threads x 4 blocks or 128 x 8 per SM).
 
 Each probe is timed with CUDA events after one untimed render; the measured table is returned
 with the choice so callers can report it.

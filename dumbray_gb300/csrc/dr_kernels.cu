@@ -91,10 +91,15 @@ __device__ __forceinline__ int warp_fetch(int *counter) {
     return __shfl_sync(0xFFFFFFFFu, base, 0);
 }
 
-// Chunked work fetch from a device counter (warp-uniform).  The chunk shrinks with the queue:
-// about 4 chunks per resident warp (152 SMs x 24 warps), between 32 and kChunk rays, so short
-// queues (late bounces, shadow queues) still spread over every resident warp.
-__device__ __forceinline__ int chunk_for(int n) { return max(32, min(kChunk, (n / (152 * 24 * 4)) & ~31)); }
+// Chunked work fetch from a device counter (warp-uniform).  The chunk shrinks with the queue: about 4
+// chunks per resident warp, between 32 and kChunk rays, and the rays of one warp when there are not
+// enough for all lanes (warp_width), so short queues (late bounces, shadow queues) still spread over
+// every resident warp.
+__device__ __forceinline__ int grid_warps() { return (int)(gridDim.x * (blockDim.x >> 5)); }
+__device__ __forceinline__ int chunk_for(int n) {
+    const int warps = grid_warps(), width = warp_width(n, warps);
+    return width < 32 ? width : max(32, min(kChunk, (n / (4 * warps)) & ~31));
+}
 __device__ __forceinline__ bool fetch_chunk(int *counter, int n, int chunk, int &b, int &e) {
     int base = 0;
     if ((threadIdx.x & 31u) == 0) base = atomicAdd(counter, chunk);
@@ -125,23 +130,25 @@ __device__ __forceinline__ void accum_add(float *acc, int slot, c3 c) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// dr_cast: warp w of the grid owns rays [w * kChunk, (w + 1) * kChunk) of one scene.
+// dr_cast: warp w of the grid traces rays [w c, (w + 1) c), then the same of every next grid's worth
+// (c = 32, or fewer when the rays do not fill the lanes).  Neighbouring rays stay together, a warp
+// refills its lanes until its last chunk, and no counter has to be cleared or kept between calls.
 struct BatchSource {
     static constexpr float kOccludeBelow = 0.0f;
     const float *o, *d;
     const int *ignore;
     int *hit_tri, *nbox, *ntri;
     float *hit_t;
-    int n;
-    bool given, cull;
+    int n, chunk;
+    long long at;         // the warp's next chunk
+    bool cull;
     const Scene *scene0;  // unused: single-scene source
     __device__ __forceinline__ bool next(int &b, int &e) {
-        if (given) return false;
-        given = true;
-        int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-        b = w * kChunk;
-        e = min(b + kChunk, n);
-        return b < n;
+        if (at >= n) return false;
+        b = (int)at;
+        e = min(b + chunk, n);
+        at += (long long)grid_warps() * chunk;
+        return true;
     }
     __device__ __forceinline__ bool load(int i, f3 &ro, f3 &rd, int &ign, int &job) {
         ro = mkf3(o[3 * i], o[3 * i + 1], o[3 * i + 2]);
@@ -165,14 +172,20 @@ struct BatchSource {
     }
 };
 
+constexpr int kCastThreads = 64;
+// 64 registers, 32 warps per SM; the counting traversal needs 80.
+constexpr int cast_blocks_per_sm(bool count) { return count ? 12 : 16; }
+
 template <bool COUNT>
-__global__ void __launch_bounds__(128) k_cast(Scene S, const float *__restrict__ o, const float *__restrict__ d,
-                                              const int *__restrict__ ignore, int n, int clip, int *__restrict__ hit_tri,
-                                              float *__restrict__ hit_t, int *__restrict__ nbox, int *__restrict__ ntri) {
+__global__ void __launch_bounds__(kCastThreads, cast_blocks_per_sm(COUNT))
+    k_cast(Scene S, const float *__restrict__ o, const float *__restrict__ d, const int *__restrict__ ignore, int n, int clip,
+           int *__restrict__ hit_tri, float *__restrict__ hit_t, int *__restrict__ nbox, int *__restrict__ ntri) {
     typename StackOf<COUNT>::type stack[kStack];
-    __shared__ WarpSlots slots[4];
-    BatchSource src{o, d, ignore, hit_tri, COUNT ? nbox : nullptr, COUNT ? ntri : nullptr, hit_t, n, false, clip != 0, &S};
-    trace_persistent<COUNT, false>(S, src, stack, slots[threadIdx.x >> 5]);
+    __shared__ WarpSlots slots[kCastThreads / 32];
+    const int width = warp_width(n, grid_warps());
+    const long long warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    BatchSource src{o, d, ignore, hit_tri, COUNT ? nbox : nullptr, COUNT ? ntri : nullptr, hit_t, n, width, warp * width, clip != 0, &S};
+    trace_persistent<COUNT, false>(S, src, stack, slots[threadIdx.x >> 5], width);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -398,15 +411,15 @@ struct TraceSource {
     }
 };
 
-// Block shape of the traversal kernels (k_trace, k_shadow_phys): 8 warps, 3 blocks per SM caps
-// registers at 80 (24 warps per SM); the traversal state needs about that many without spilling.
-// Measured on the 1080p path trace (Mpaths/s): 256x3 205.7, 128x6 205.4 (80 registers), 128x7 199.8
-// and 64x13 199.8 (72 registers, spills).
+// Block shape of the traversal kernels (k_trace, k_shadow_phys, k_shadow_ref): 8 warps, 4 blocks per SM
+// cap registers at 64 (32 warps per SM), which the traversal state fits without spilling.  4 against 3
+// blocks (80 registers), in one call: room 9.40 -> 8.67 ms, 1080p photon render 44.2 -> 42.1 ms, path
+// trace 38.4 -> 35.7 ms, gradients 73.0 -> 70.4 ms.
 constexpr int kTraceThreads = 256;
-constexpr int kTraceBlocksPerSM = 3;
+constexpr int kTraceBlocksPerSM = 4;
 
-// Block shapes a renderer can select (dr_renderer_set_block_shape): 0 = 256 x 3, 1 = 128 x 6 per SM
-// (both cap registers at 80); the autotuner times them.
+// Block shapes a renderer can select (dr_renderer_set_block_shape): 0 = 256 x 4, 1 = 128 x 8 per SM
+// (both cap registers at 64); the autotuner times them.
 template <bool COUNT, bool MULTI, int TT = kTraceThreads, int TB = kTraceBlocksPerSM>
 __global__ void __launch_bounds__(TT, TB) k_trace(WaveArgs A, int b) {
     Ctrl *C = A.ctrl;
@@ -414,7 +427,7 @@ __global__ void __launch_bounds__(TT, TB) k_trace(WaveArgs A, int b) {
     typename StackOf<COUNT>::type stack[kStack];
     __shared__ WarpSlots slots[TT / 32];
     TraceSource<MULTI> src{&A, A.q[b & 1], A.hits, &C->fetch_trace[b], n, chunk_for(n), 0, 0, 0};
-    trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], A.inl.S.front_only ? kPhysStepsPerRound : 1);
+    trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], warp_width(n, grid_warps()), A.inl.S.front_only ? kPhysStepsPerRound : 1);
     if (COUNT) count_add64(A.counters, src.rays, src.nb, src.nt);
 }
 
@@ -683,7 +696,7 @@ struct RefPhotonChainSource {
 // Blocks per SM of the photon kernels (kTraceThreads threads each): the first-cast kernel holds no
 // shading and takes the traversal's own budget; the chain kernel, with the blocker shading, gets up
 // to 128 registers.
-constexpr int kShadowRefBlocksPerSM = 3;
+constexpr int kShadowRefBlocksPerSM = 4;
 constexpr int kPhotonChainBlocksPerSM = 2;
 
 template <bool COUNT, bool MULTI>
@@ -695,7 +708,7 @@ __global__ void __launch_bounds__(kTraceThreads, kShadowRefBlocksPerSM) k_shadow
     __shared__ WarpSlots slots[kTraceThreads / 32];
     RefPhotonSource<MULTI> src{&A, A.sq, &C->fetch_shadow[b], &C->carry_count, blocked_list(A, b), &C->blocked_count[b], n,
                                chunk_for(n), 0, 0, 0};
-    trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5]);
+    trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], warp_width(n, grid_warps()));
     if (COUNT) count_add64(A.counters + 3, src.rays, src.nb, src.nt);
 }
 
@@ -711,7 +724,7 @@ __global__ void __launch_bounds__(kTraceThreads, kPhotonChainBlocksPerSM) k_phot
     __shared__ WarpSlots slots[kTraceThreads / 32];
     RefPhotonChainSource<MULTI> src{&A, carry ? A.cq : A.sq, carry ? nullptr : blocked_list(A, b),
                                     carry ? &C->fetch_carry : &C->fetch_chain[b], n, chunk_for(n), 0, 0, 0};
-    trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5]);
+    trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], warp_width(n, grid_warps()));
     if (COUNT) count_add64(A.counters + 3, src.rays, src.nb, src.nt);
 }
 
@@ -994,7 +1007,7 @@ __global__ void __launch_bounds__(TT, TB) k_shadow_phys(WaveArgs A, int b) {
     typename StackOf<COUNT>::type stack[kStack];
     __shared__ WarpSlots slots[TT / 32];
     ShadowPhysSource<MULTI, ADJ> src{&A, A.sq, A.accum, &C->fetch_shadow[b], n, chunk_for(n), 0, 0, 0};
-    trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], A.inl.S.front_only ? kPhysStepsPerRound : 1);
+    trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], warp_width(n, grid_warps()), A.inl.S.front_only ? kPhysStepsPerRound : 1);
     if (COUNT) count_add64(A.counters + 3, src.rays, src.nb, src.nt);
 }
 
@@ -1131,13 +1144,13 @@ static int sm_count() {
 cudaError_t launch_cast(const Scene &S, const float *o, const float *d, const int *ignore, int n, int clip, int *hit_tri,
                         float *hit_t, int *nbox, int *ntri, cudaStream_t stream, long long *launches) {
     if (n <= 0) return cudaSuccess;
-    int threads = 128;
-    int per_block = (threads / 32) * kChunk;
-    int blocks = (n + per_block - 1) / per_block;
+    // one warp per ray until the resident warps are used up
+    const int blocks = (int)std::min<long long>((n + kCastThreads / 32 - 1) / (kCastThreads / 32),
+                                                (long long)sm_count() * cast_blocks_per_sm(nbox || ntri));
     if (nbox || ntri)
-        k_cast<true><<<blocks, threads, 0, stream>>>(S, o, d, ignore, n, clip, hit_tri, hit_t, nbox, ntri);
+        k_cast<true><<<blocks, kCastThreads, 0, stream>>>(S, o, d, ignore, n, clip, hit_tri, hit_t, nbox, ntri);
     else
-        k_cast<false><<<blocks, threads, 0, stream>>>(S, o, d, ignore, n, clip, hit_tri, hit_t, nullptr, nullptr);
+        k_cast<false><<<blocks, kCastThreads, 0, stream>>>(S, o, d, ignore, n, clip, hit_tri, hit_t, nullptr, nullptr);
     if (launches) (*launches)++;
     return cudaGetLastError();
 }
@@ -1274,7 +1287,7 @@ static void launch_wave_t(const WaveDesc &W, const WaveArgs &A, cudaStream_t str
     k_camera<MULTI><<<grid, 256, 0, stream>>>(A);
     P.end(KC_CAMERA, stream);
     nl++;
-    const int tgrid = grid * (256 / TT);   // same threads in flight as the 256-thread kernels
+    const int tgrid = sm_count() * TB;   // one persistent block per slot
     for (int b = 0; b <= W.max_bounces; b++) {
         P.begin(KC_TRACE, stream);
         if (count) k_trace<true, MULTI, TT, TB><<<tgrid, TT, 0, stream>>>(A, b);
@@ -1329,8 +1342,8 @@ cudaError_t launch_wave(const WaveDesc &W, cudaStream_t stream, long long *launc
     Profiler &P = prof ? *prof : dummy;
     const bool cnt = counters != nullptr;
     if (W.shape == 1) {
-        if (W.items) launch_wave_t<true, 128, 6>(W, A, stream, P, cnt, nl);
-        else launch_wave_t<false, 128, 6>(W, A, stream, P, cnt, nl);
+        if (W.items) launch_wave_t<true, 128, 8>(W, A, stream, P, cnt, nl);
+        else launch_wave_t<false, 128, 8>(W, A, stream, P, cnt, nl);
     } else {
         if (W.items) launch_wave_t<true, kTraceThreads, kTraceBlocksPerSM>(W, A, stream, P, cnt, nl);
         else launch_wave_t<false, kTraceThreads, kTraceBlocksPerSM>(W, A, stream, P, cnt, nl);
