@@ -129,6 +129,13 @@ __device__ __forceinline__ void accum_add(float *acc, int slot, c3 c) {
     if (c.b != 0.0f) atomicAdd(acc + 4 * slot + 2, c.b);
 }
 
+// Traversal steps a lane may take between two leaf rounds.  Same call, 1 / 2 / 3 / 4 steps.  Reference
+// tree: room 8.74 / 8.13 / - ms, 1080p photon render 41.3 / 38.3 / 38.9 ms, primary casts 1.18 / 1.19 /
+// 1.24 ms.  Physical tree, whose leaves are smaller: 8.4M incoherent casts 3.32 / 2.92 / 2.85 / 2.83 ms,
+// path trace - / 35.4 / 34.8 / 34.2 ms, batch - / 12.12 / 11.91 / 12.02 ms, gradients - / 69.5 / 69.5 /
+// 70.5 ms.
+__host__ __device__ constexpr int steps_per_round(bool physical) { return physical ? 3 : 2; }
+
 // ---------------------------------------------------------------------------------------------
 // dr_cast: warp w of the grid traces rays [w c, (w + 1) c), then the same of every next grid's worth
 // (c = 32, or fewer when the rays do not fill the lanes).  Neighbouring rays stay together, a warp
@@ -185,7 +192,7 @@ __global__ void __launch_bounds__(kCastThreads, cast_blocks_per_sm(COUNT))
     const int width = warp_width(n, grid_warps());
     const long long warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     BatchSource src{o, d, ignore, hit_tri, COUNT ? nbox : nullptr, COUNT ? ntri : nullptr, hit_t, n, width, warp * width, clip != 0, &S};
-    trace_persistent<COUNT, false>(S, src, stack, slots[threadIdx.x >> 5], width);
+    trace_persistent<COUNT, false>(S, src, stack, slots[threadIdx.x >> 5], width, steps_per_round(S.front_only != 0));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -371,12 +378,6 @@ __global__ void __launch_bounds__(256) k_camera(WaveArgs A) {
     }
 }
 
-// Traversal steps a lane may take between two cooperative leaf rounds on physical-tree scenes
-// (small leaves; the reference's tree keeps 1).  Path trace of the open 1.31M-triangle scene at leaf
-// split 4, Mpaths/s: 1: 654, 2: 789, 3: 795, 4: 810, 6: 723, 8: 648; but 4 slowed the closed scenes
-// (box rooms: adjoint forward 43.5 -> 51.5 ms, 64-scene batch 405 -> 378 Mpaths/s), so it stays 2.
-constexpr int kPhysStepsPerRound = 2;
-
 template <bool MULTI>
 struct TraceSource {
     static constexpr float kOccludeBelow = 0.0f;
@@ -427,7 +428,8 @@ __global__ void __launch_bounds__(TT, TB) k_trace(WaveArgs A, int b) {
     typename StackOf<COUNT>::type stack[kStack];
     __shared__ WarpSlots slots[TT / 32];
     TraceSource<MULTI> src{&A, A.q[b & 1], A.hits, &C->fetch_trace[b], n, chunk_for(n), 0, 0, 0};
-    trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], warp_width(n, grid_warps()), A.inl.S.front_only ? kPhysStepsPerRound : 1);
+    trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], warp_width(n, grid_warps()),
+                                   steps_per_round(A.inl.S.front_only != 0));
     if (COUNT) count_add64(A.counters, src.rays, src.nb, src.nt);
 }
 
@@ -708,7 +710,8 @@ __global__ void __launch_bounds__(kTraceThreads, kShadowRefBlocksPerSM) k_shadow
     __shared__ WarpSlots slots[kTraceThreads / 32];
     RefPhotonSource<MULTI> src{&A, A.sq, &C->fetch_shadow[b], &C->carry_count, blocked_list(A, b), &C->blocked_count[b], n,
                                chunk_for(n), 0, 0, 0};
-    trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], warp_width(n, grid_warps()));
+    trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], warp_width(n, grid_warps()),
+                                   steps_per_round(A.inl.S.front_only != 0));
     if (COUNT) count_add64(A.counters + 3, src.rays, src.nb, src.nt);
 }
 
@@ -724,7 +727,8 @@ __global__ void __launch_bounds__(kTraceThreads, kPhotonChainBlocksPerSM) k_phot
     __shared__ WarpSlots slots[kTraceThreads / 32];
     RefPhotonChainSource<MULTI> src{&A, carry ? A.cq : A.sq, carry ? nullptr : blocked_list(A, b),
                                     carry ? &C->fetch_carry : &C->fetch_chain[b], n, chunk_for(n), 0, 0, 0};
-    trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], warp_width(n, grid_warps()));
+    trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], warp_width(n, grid_warps()),
+                                   steps_per_round(A.inl.S.front_only != 0));
     if (COUNT) count_add64(A.counters + 3, src.rays, src.nb, src.nt);
 }
 
@@ -1007,7 +1011,8 @@ __global__ void __launch_bounds__(TT, TB) k_shadow_phys(WaveArgs A, int b) {
     typename StackOf<COUNT>::type stack[kStack];
     __shared__ WarpSlots slots[TT / 32];
     ShadowPhysSource<MULTI, ADJ> src{&A, A.sq, A.accum, &C->fetch_shadow[b], n, chunk_for(n), 0, 0, 0};
-    trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], warp_width(n, grid_warps()), A.inl.S.front_only ? kPhysStepsPerRound : 1);
+    trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], warp_width(n, grid_warps()),
+                                   steps_per_round(A.inl.S.front_only != 0));
     if (COUNT) count_add64(A.counters + 3, src.rays, src.nb, src.nt);
 }
 

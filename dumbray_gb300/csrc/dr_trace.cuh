@@ -166,13 +166,12 @@ __device__ __forceinline__ int warp_width(int n, int warps) { return max(1, min(
 constexpr int kRoundBits = 5;
 constexpr int kRoundCap = (1 << kRoundBits) - 1;
 
-// steps_per_round: traversal steps a lane may take between two leaf rounds while it stays in inner
-// nodes; more means fewer rounds, but lanes that reached a leaf wait longer (measured: 2 pays on
-// physical-tree scenes, whose leaves are small; 1 elsewhere).
+// steps: traversal steps a lane may take between two leaf rounds while it stays in inner nodes; more
+// means fewer rounds, but lanes that reached a leaf wait longer.
 // width: lanes that take rays (see warp_width); all 32 test triangles.
 template <bool COUNT, bool MULTI, class Source>
 __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, typename StackOf<COUNT>::type *stack, WarpSlots &ws,
-                                                 int width, int steps_per_round = 1) {
+                                                 int width, int steps) {
     constexpr unsigned kAll = 0xFFFFFFFFu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt_mask = (1u << lane) - 1u;
@@ -228,7 +227,7 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ty
             continue;
         }
 #pragma unroll 1
-        for (int step = 0; step < steps_per_round; step++) {
+        for (int step = 0; step < steps; step++) {
             if (mode != kTrav) break;
             // ---- one traversal step: pop an empty frame, then take one child
             if constexpr (COUNT) {
