@@ -1084,6 +1084,7 @@ dr_status dr_render_blocks(dr_renderer *r, const dr_scene *sc, const dr_camera *
     W.adjoint = false;
     wave_buffers(r, W);
     const int lights = (I.mode == DR_MODE_REFERENCE) ? I.S.shadow_photons : 1;
+    W.photons = lights;
     const long long total = (long long)I.n_slots * I.spp;
     const long long wave = lane_wave(total, wave_size(r, lights, 1LL << 40), r->lanes);
     return run_waves(r, W, total, wave, I.n_slots, stream, &r->prof, r->counting, true, r->lanes);
@@ -1329,6 +1330,7 @@ dr_status dr_batch_render(dr_renderer *r, dr_batch *b, int32_t use_graph, void *
     W.n_items = (int)b->items.size();
     W.mode = b->mode;
     W.max_bounces = b->max_bounces;
+    W.photons = b->max_lights;
     W.adjoint = false;
     wave_buffers(r, W);
     const long long wave = lane_wave(b->total_paths, wave_size(r, b->mode == DR_MODE_REFERENCE ? b->max_lights : 1, 1LL << 40),

@@ -6,7 +6,8 @@
 //   k_shade_ref       DumbRenderer layer step (DumbRenderer.cu:249-443) as one forward path step:
 //                     indirect request, light photons -> shadow queue, next ray -> next queue
 //   k_shadow_ref      light -> point visibility, first cast of every photon (DumbRenderer.cu:361-428)
-//   k_photon_chain    photons stopped by a blocker: the reference's transparency re-casts
+//   k_photon_filter   photons stopped by a blocker: which of them the blocker lets continue
+//   k_photon_chain    those that continue: the reference's transparency re-casts
 //   k_shade_phys      physical path step (emission + MIS, NEE -> shadow queue, BSDF sample);
 //                     in the adjoint pass it also scatters gradients of emission hits
 //   k_shadow_phys     point -> light visibility; in the adjoint pass it marks the visible records
@@ -203,9 +204,10 @@ struct Ctrl {
     int fetch_trace[kMaxBounceSlots];
     int fetch_shade[kMaxBounceSlots];
     int fetch_shadow[kMaxBounceSlots];
-    int blocked_count[kMaxBounceSlots];   // reference photons stopped by a blocker at bounce b and
-    int fetch_chain[kMaxBounceSlots];     // left in place (the carry region was full)
-    int carry_count;                      // blocked reference photons moved to the carry region
+    int blocked_count[kMaxBounceSlots];   // reference photons stopped by a blocker at bounce b
+    int fetch_chain[kMaxBounceSlots];
+    int kept_count[kMaxBounceSlots];      // those of them that continue when the carry region is full
+    int carry_count;                      // continuing reference photons moved to the carry region
     int fetch_carry;
     int fetch_camera;
     int error;
@@ -236,7 +238,8 @@ struct WaveArgs {
     float2 *hits;
     ShadowQ sq;
     ShadowQ cq;             // carry region of the shadow planes (blocked reference photons)
-    int carry_cap;
+    int carry_cap, shadow_cap;
+    bool roomy;             // the carry region holds every photon of the wave
     float *accum;           // [total slots][4]
     Ctrl *ctrl;
     unsigned long long *counters;  // counting pass only
@@ -544,19 +547,23 @@ __global__ void __launch_bounds__(kShadeThreads) k_shade_ref(WaveArgs A, int b) 
 // point; otherwise the blocker's reflected colour decides whether the photon continues (from just
 // past the blocker, with that colour, the blocker as the ignored object).
 //
-// The casts run on the persistent traversal engine.  k_shadow_ref casts every photon of a bounce
-// once and settles those that arrive or miss; a photon stopped by a blocker becomes a blocked record
-// (the hit point in s0, the blocker in s2.w, its cast count negated in s3.w) in the wave's carry
-// region.  k_photon_chain, once per wave after the last bounce, takes the blocked photons: the
-// blocker's colour decides whether each continues, and a continuing photon starts its next cast at
-// once in the same lane (its record rewritten in place, the engine's restart), so a chain of any
-// length keeps its lane.  Under 1% of the photons of the path-trace twin are ever blocked, but
-// compiled into the cast kernel the blocker shading and the chain restart cost every cast, and a
-// chain launch per bounce would end every bounce with its longest chain; so the cast kernel holds
-// no shading code and the chains wait for the wave's end.  When the carry region is full a blocked
-// photon stays in its bounce's record and joins the bounce's blocked list (in the spent extension
-// queue), which a k_photon_chain launch right after the bounce's casts takes (an empty launch
-// otherwise).  Chains read nothing that later bounces write, so neither order changes a result.
+// The casts run on the persistent traversal engine.  k_shadow_ref casts every photon of a bounce once
+// and settles those that arrive or miss; a photon stopped by a blocker stays in its record (the hit
+// point in s0, the blocker in s2.w, its cast count negated in s3.w) and joins the bounce's blocked list
+// (in the spent extension queue).  k_photon_filter shades the blockers, one thread per photon: nearly
+// all end there (a DumbBased surface met from its front passes nothing), and those that continue move
+// to the wave's carry region as their next cast.  k_photon_chain, once per wave after the last bounce,
+// runs the carried photons' chains: a photon that continues again starts its next cast at once in the
+// same lane (its record rewritten in place, the engine's restart).  When the carry region is full a
+// photon joins the bounce's kept list instead, which a k_photon_chain launch right after takes (an
+// empty launch otherwise).  A wave whose photons all fit into the carry region (`roomy`, known from its
+// size) needs neither launch: its blocked photons are carried unshaded and shaded as their chain begins,
+// which saves two of a small wave's five launches a bounce.  Chains read nothing that later bounces
+// write, so no order changes a result.  Shading stays out of the cast kernel, whose registers are the
+// traversal's, and a launch of long chains out of every bounce.
+// Carrying every wave's blocked photons unshaded filled the carry region where a third of the photons
+// meet a shadowed side, and every bounce ended with a chain launch of 0.15-0.70 ms: 1080p photon render
+// of 2x2 samples 39.0 -> 35.5 ms with the filter, same call.
 // At most kPhotonCasts casts per photon (the oracle's bound, never reached by a photon that moves
 // along one line through finite geometry); the count travels in s3.w.
 constexpr int kPhotonCasts = 64;
@@ -570,10 +577,11 @@ __device__ __forceinline__ bool photon_arrives(const Hit &h, int target, f3 hp) 
 // registers do not weigh on the traversal it is reached from.
 __device__ __noinline__ c3 blocker_reflect(const Scene &S, int tri, f3 p, f3 ld) { return ref_reflect(S, tri, p, ld, ld, true, 0); }
 
-// Blocked photon lists live in the bounce's spent extension queue: in reference mode nothing reads
-// q[b & 1] between k_shade_ref(b) and k_shade_ref(b + 1), and its p0 plane (4 ints per path) holds
-// the bounce's photons (at most 2 per path of the wave's capacity).
+// The lists live in the bounce's spent extension queue: in reference mode nothing reads q[b & 1]
+// between k_shade_ref(b) and k_shade_ref(b + 1), and its p0 plane (4 ints per path) holds two lists of
+// the bounce's photons (at most shadow_cap = 2 per path of the wave's capacity).
 __device__ __forceinline__ int *blocked_list(const WaveArgs &A, int b) { return reinterpret_cast<int *>(A.q[b & 1].p0); }
+__device__ __forceinline__ int *kept_list(const WaveArgs &A, int b) { return blocked_list(A, b) + A.shadow_cap; }
 
 // Photon j, stopped by blocker `tri` at `p` after `casts` casts: the blocker's reflected colour
 // decides whether it continues; if so its record becomes the next cast.  False: the photon ends.
@@ -633,42 +641,66 @@ struct RefPhotonSource {
         const float4 s3 = sq.s3[i];
         const int casts = __float_as_int(s3.w) + 1;
         if (casts >= kPhotonCasts) return false;
-        const float4 b0 = make_float4(h.p.x, h.p.y, h.p.z, sq.s0[i].w);
-        const float4 b2 = make_float4(s2.x, s2.y, s2.z, __int_as_float(h.tri));
-        const float4 b3 = make_float4(s3.x, s3.y, s3.z, __int_as_float(-casts));
-        const int k = atomicAdd(carry_count, 1);
-        if (k < A->carry_cap) {
+        const float4 s0 = make_float4(h.p.x, h.p.y, h.p.z, sq.s0[i].w);
+        if (A->roomy) {
             const ShadowQ &cq = A->cq;
-            cq.s0[k] = b0;
+            const int k = atomicAdd(carry_count, 1);
+            cq.s0[k] = s0;
             cq.s1[k] = sq.s1[i];
-            cq.s2[k] = b2;
-            cq.s3[k] = b3;
+            cq.s2[k] = make_float4(s2.x, s2.y, s2.z, __int_as_float(h.tri));
+            cq.s3[k] = make_float4(s3.x, s3.y, s3.z, __int_as_float(-casts));
             cq.s4[k] = sq.s4[i];
         } else {
-            sq.s0[i] = b0;
-            sq.s2[i] = b2;
-            sq.s3[i] = b3;
+            sq.s0[i] = s0;
+            sq.s2[i] = make_float4(s2.x, s2.y, s2.z, __int_as_float(h.tri));
+            sq.s3[i] = make_float4(s3.x, s3.y, s3.z, __int_as_float(-casts));
             blocked[atomicAdd(blocked_count, 1)] = i;
         }
         return false;
     }
 };
 
-// Blocked photons and their chains (k_photon_chain): entry i is record blocked[i] of `sq` (a
-// bounce's records), or record i when `blocked` is null (the carry region).
+// Which of a bounce's blocked photons continue, one thread each.
+template <bool MULTI>
+__global__ void __launch_bounds__(256) k_photon_filter(WaveArgs A, int b) {
+    Ctrl *C = A.ctrl;
+    const int n = *((volatile int *)&C->blocked_count[b]);
+    const int *blocked = blocked_list(A, b);
+    int *kept = kept_list(A, b);
+    const ShadowQ &sq = A.sq, &cq = A.cq;
+    for (int base = (int)(blockIdx.x * blockDim.x); base < n; base += (int)(gridDim.x * blockDim.x)) {
+        const int i = base + (int)threadIdx.x;
+        const int j = i < n ? blocked[i] : 0;
+        const bool on = i < n && photon_pass<MULTI>(A, sq, j, __float_as_int(sq.s2[j].w), f3of(sq.s0[j]), -__float_as_int(sq.s3[j].w));
+        const int k = warp_alloc(&C->carry_count, on);
+        if (!on) continue;
+        if (k < A.carry_cap) {
+            cq.s0[k] = sq.s0[j];
+            cq.s1[k] = sq.s1[j];
+            cq.s2[k] = sq.s2[j];
+            cq.s3[k] = sq.s3[j];
+            cq.s4[k] = sq.s4[j];
+        } else {
+            kept[atomicAdd(&C->kept_count[b], 1)] = j;
+        }
+    }
+}
+
+// Continuing photons and their chains (k_photon_chain): entry i is record kept[i] of `sq` (a bounce's
+// records), or record i when `kept` is null (the carry region).
 template <bool MULTI>
 struct RefPhotonChainSource {
     static constexpr float kOccludeBelow = 0.0f;
     const WaveArgs *A;
     ShadowQ sq;
-    const int *blocked;
+    const int *kept;
     int *fetch;
     int n, chunk;
     long long rays, nb, nt;
     __device__ __forceinline__ bool next(int &b, int &e) { return fetch_chunk(fetch, n, chunk, b, e); }
     __device__ __forceinline__ bool load(int i, f3 &o, f3 &d, int &ign, int &job) {
-        const int j = blocked ? blocked[i] : i;
-        const int w = __float_as_int(sq.s3[j].w);
+        const int j = kept ? kept[i] : i;
+        const int w = __float_as_int(sq.s3[j].w);   // negative: a roomy wave's photon, not shaded yet
         if (w < 0 && !photon_pass<MULTI>(*A, sq, j, __float_as_int(sq.s2[j].w), f3of(sq.s0[j]), -w)) return false;
         o = f3of(sq.s0[j]);
         d = f3of(sq.s1[j]);
@@ -676,7 +708,7 @@ struct RefPhotonChainSource {
         job = __float_as_int(sq.s4[j].w);
         return true;
     }
-    __device__ __forceinline__ int job(int i) { return __float_as_int(sq.s4[blocked ? blocked[i] : i].w); }
+    __device__ __forceinline__ int job(int i) { return __float_as_int(sq.s4[kept ? kept[i] : i].w); }
     __device__ __forceinline__ const Scene &scene(int job) { return job_of<MULTI>(*A, job).S; }
     __device__ __forceinline__ bool clip(int job) { return job_of<MULTI>(*A, job).clip != 0; }
     __device__ __forceinline__ bool store(int i, const Hit &h, int b_, int t_) {
@@ -684,7 +716,7 @@ struct RefPhotonChainSource {
         nb += b_;
         nt += t_;
         if (h.tri < 0) return false;
-        const int j = blocked ? blocked[i] : i;
+        const int j = kept ? kept[i] : i;
         if (photon_arrives(h, __float_as_int(sq.s1[j].w), f3of(sq.s2[j]))) {
             photon_arrive(*A, sq, j);
             return false;
@@ -715,17 +747,17 @@ __global__ void __launch_bounds__(kTraceThreads, kShadowRefBlocksPerSM) k_shadow
     if (COUNT) count_add64(A.counters + 3, src.rays, src.nb, src.nt);
 }
 
-// b >= 0: bounce b's blocked list (photons the full carry region turned away); b < 0: the carry
+// b >= 0: bounce b's kept list (photons the full carry region turned away); b < 0: the carry
 // region, after the wave's last bounce.
 template <bool COUNT, bool MULTI>
 __global__ void __launch_bounds__(kTraceThreads, kPhotonChainBlocksPerSM) k_photon_chain(WaveArgs A, int b) {
     Ctrl *C = A.ctrl;
     const bool carry = b < 0;
-    const int n = carry ? min(*((volatile int *)&C->carry_count), A.carry_cap) : *((volatile int *)&C->blocked_count[b]);
+    const int n = carry ? min(*((volatile int *)&C->carry_count), A.carry_cap) : *((volatile int *)&C->kept_count[b]);
     if (n == 0) return;
     typename StackOf<COUNT>::type stack[kStack];
     __shared__ WarpSlots slots[kTraceThreads / 32];
-    RefPhotonChainSource<MULTI> src{&A, carry ? A.cq : A.sq, carry ? nullptr : blocked_list(A, b),
+    RefPhotonChainSource<MULTI> src{&A, carry ? A.cq : A.sq, carry ? nullptr : kept_list(A, b),
                                     carry ? &C->fetch_carry : &C->fetch_chain[b], n, chunk_for(n), 0, 0, 0};
     trace_persistent<COUNT, MULTI>(A.inl.S, src, stack, slots[threadIdx.x >> 5], warp_width(n, grid_warps()),
                                    steps_per_round(A.inl.S.front_only != 0));
@@ -1333,6 +1365,8 @@ static void fill_args(const WaveDesc &W, WaveArgs &A, unsigned long long *counte
     A.sq.s3 = W.s[3];
     A.sq.s4 = W.s[4];
     A.carry_cap = carry_capacity(W.shadow_cap);
+    A.shadow_cap = W.shadow_cap;
+    A.roomy = (long long)W.wave_count * (W.max_bounces + 1) * W.photons <= A.carry_cap;
     A.cq.s0 = W.s[0] + W.shadow_cap;
     A.cq.s1 = W.s[1] + W.shadow_cap;
     A.cq.s2 = W.s[2] + W.shadow_cap;
@@ -1366,14 +1400,14 @@ static void launch_wave_t(const WaveDesc &W, const WaveArgs &A, cudaStream_t str
         if (W.mode == DR_MODE_REFERENCE) {
             const int sgrid = sm_count() * kShadowRefBlocksPerSM;   // one persistent block per slot
             const int cgrid = sm_count() * kPhotonChainBlocksPerSM;
-            if (count) {
-                k_shadow_ref<true, MULTI><<<sgrid, kTraceThreads, 0, stream>>>(A, b);
-                k_photon_chain<true, MULTI><<<cgrid, kTraceThreads, 0, stream>>>(A, b);
-            } else {
-                k_shadow_ref<false, MULTI><<<sgrid, kTraceThreads, 0, stream>>>(A, b);
-                k_photon_chain<false, MULTI><<<cgrid, kTraceThreads, 0, stream>>>(A, b);
+            if (count) k_shadow_ref<true, MULTI><<<sgrid, kTraceThreads, 0, stream>>>(A, b);
+            else k_shadow_ref<false, MULTI><<<sgrid, kTraceThreads, 0, stream>>>(A, b);
+            if (!A.roomy) {
+                k_photon_filter<MULTI><<<grid, 256, 0, stream>>>(A, b);
+                if (count) k_photon_chain<true, MULTI><<<cgrid, kTraceThreads, 0, stream>>>(A, b);
+                else k_photon_chain<false, MULTI><<<cgrid, kTraceThreads, 0, stream>>>(A, b);
+                nl += 2;
             }
-            nl++;
         } else if (!MULTI && W.adjoint) {
             k_shadow_phys<false, false, true, TT, TB><<<tgrid, TT, 0, stream>>>(A, b);
             k_adj_shadow<<<sm_count() * 4, 256, 0, stream>>>(A, b);

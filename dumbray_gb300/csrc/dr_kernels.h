@@ -11,7 +11,7 @@ namespace drd {
 constexpr int kMaxBounceSlots = 68;  // bounce limit 64 (DUMB_RENDERER_BOUNCE_LIMIT) + camera + spare
 constexpr int kAdjDepth = 66;        // prefix slots per path in the adjoint pass (bounces 0..64)
 
-// Reference photons stopped by a blocker wait for their transparency chains in a carry region of
+// Reference photons that go on past a blocker wait for their transparency chains in a carry region of
 // the shadow planes, behind the `shadow_cap` photon records of a bounce, until the end of the wave.
 constexpr int carry_capacity(int shadow_cap) { return std::max(1024, (shadow_cap / 16 + 31) / 32 * 32); }
 constexpr size_t shadow_plane_records(int shadow_cap) { return (size_t)shadow_cap + (size_t)carry_capacity(shadow_cap); }
@@ -46,6 +46,7 @@ struct WaveDesc {
     const Item *items;           // device job table (batches) or nullptr
     int n_items;
     int mode, max_bounces;
+    int photons;                 // reference mode: most photon records one hit can emit
     long long wave_begin;
     int wave_count;
     float4 *q_p0[2], *q_p1[2], *q_p2[2];

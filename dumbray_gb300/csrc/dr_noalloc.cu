@@ -118,6 +118,7 @@ extern "C" dr_status dr_render_blocks_noalloc(const dr_scene *sc, const dr_camer
     W.n_items = 1;
     W.mode = p->mode;
     W.max_bounces = p->max_bounces;
+    W.photons = per_path_shadow;
     W.adjoint = false;
     for (int k = 0; k < 2; k++) {
         W.q_p0[k] = reinterpret_cast<float4 *>(base + kOffQueues + (4 * k + 0) * kQueuePlane);
