@@ -288,14 +288,30 @@ constexpr int kCountShift = 11;
 // What bounds it is instruction issue (55-69% of the issue slots at 15-17 of 32 lanes) and the wait for
 // the record; against the exact test on nodes and planes, in one call: 8.4M incoherent casts on the
 // 1.31M-triangle mesh 5.02 -> 4.34 ms, the 1080p 16 spp path trace 48.9 -> 44.2 ms, the room of 20k
-// triangles 14.4 -> 13.2 ms, 512^2 gradients 98.2 -> 87.5 ms.
+// triangles 14.4 -> 13.2 ms, 512^2 gradients 98.2 -> 87.5 ms; two children an instruction then 1-3% on
+// every case.
 constexpr int kRecordF4 = 16;
 constexpr float kRecordPad = 1.0f / 524288.0f;
 constexpr float kRaySlack = 1.0f / 1048576.0f;
 
-// What record_mask needs of a ray: 1 / d and the offsets of the near and far planes.
+// Two floats in one register pair, and a fused multiply-add of both (one issue slot on sm_100 and later).
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+// What record_mask needs of a ray: 1 / d and the negated offsets of the near and far planes, each twice
+// in a pair.
 struct RaySlopes {
-    float inv[3], near[3], far[3];
+    f32x2 inv[3], near[3], far[3];
 };
 // The direction is scaled to a largest component in [1, 2) (a power of two: exact), so only origins
 // beyond 1e24 could take a product out of the float range; such an axis is not tested (near = -max,
@@ -315,9 +331,10 @@ __device__ __forceinline__ RaySlopes ray_slopes(f3 o, f3 d, float reach) {
         const float inv = __fdiv_rn(1.0f, dc[k] < 0.0f ? -a : a);
         const float oi = oc[k] * inv, e = fabsf(oi) * kRaySlack;
         const bool ok = fabsf(inv) * (reach + fabsf(oc[k])) < 1e37f;
-        r.inv[k] = ok ? inv : 0.0f;
-        r.near[k] = ok ? oi + e : FLT_MAX;
-        r.far[k] = ok ? oi - e - eps2 : -FLT_MAX;
+        const float i = ok ? inv : 0.0f, n = ok ? -oi - e : -FLT_MAX, f = ok ? eps2 + e - oi : FLT_MAX;
+        r.inv[k] = pack2(i, i);
+        r.near[k] = pack2(n, n);
+        r.far[k] = pack2(f, f);
     }
     return r;
 }
@@ -328,36 +345,50 @@ __device__ __forceinline__ bool never_hits(f3 o, f3 d) {
     return z != 0.0f || z != z || (d.x == 0.0f && d.y == 0.0f && d.z == 0.0f);
 }
 
+__device__ __forceinline__ void ldg8(const char *p, f32x2 *v) {
+    asm("ld.global.nc.v4.b64 {%0,%1,%2,%3}, [%4];" : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(p));
+}
+
 // Children of group `g` that the ray may enter, bit k = child (order ^ k), and the group's word 48.
-// Per child: six fused multiply-adds, the interval of the three axes, and its sign bit shifted into
-// the mask.
+// Per child: six fused multiply-adds (two children an instruction), the interval of the three axes, and
+// its sign bit shifted into the mask.
 __device__ __forceinline__ unsigned record_mask(const float4 *groups, uint32_t g, int order, const RaySlopes &r, uint32_t &links) {
     const char *p = reinterpret_cast<const char *>(groups + (size_t)g * kRecordF4);
     links = __ldg(reinterpret_cast<const uint32_t *>(p + 192));
-    float mn[8], mx[8], n[8], f[8];
     const int sx = (order & 4) << 3, sy = (order & 2) << 4, sz = (order & 1) << 5;   // byte offset of the near plane: 0 or 32
-    ldg8(p + sx, mn);
-    ldg8(p + (sx ^ 32), mx);
+    f32x2 n[4], f[4];
+    float mn[8], mx[8];
+    ldg8(p + sx, n);
+    ldg8(p + (sx ^ 32), f);
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-        mn[c] = fmaxf(__fmaf_rn(mn[c], r.inv[0], -r.near[0]), 0.0f);
-        mx[c] = __fmaf_rn(mx[c], r.inv[0], -r.far[0]);
+    for (int c = 0; c < 4; c++) {
+        unpack2(fma2(n[c], r.inv[0], r.near[0]), mn[2 * c], mn[2 * c + 1]);
+        unpack2(fma2(f[c], r.inv[0], r.far[0]), mx[2 * c], mx[2 * c + 1]);
     }
     ldg8(p + 64 + sy, n);
     ldg8(p + 64 + (sy ^ 32), f);
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-        mn[c] = fmaxf(mn[c], __fmaf_rn(n[c], r.inv[1], -r.near[1]));
-        mx[c] = fminf(mx[c], __fmaf_rn(f[c], r.inv[1], -r.far[1]));
+    for (int c = 0; c < 4; c++) {
+        float a, b;
+        unpack2(fma2(n[c], r.inv[1], r.near[1]), a, b);
+        asm("max.f32 %0, %0, %1, 0f00000000;" : "+f"(mn[2 * c]) : "f"(a));   // and not behind the origin
+        asm("max.f32 %0, %0, %1, 0f00000000;" : "+f"(mn[2 * c + 1]) : "f"(b));
+        unpack2(fma2(f[c], r.inv[1], r.far[1]), a, b);
+        mx[2 * c] = fminf(mx[2 * c], a);
+        mx[2 * c + 1] = fminf(mx[2 * c + 1], b);
     }
     ldg8(p + 128 + sz, n);
     ldg8(p + 128 + (sz ^ 32), f);
     unsigned m = 0;
 #pragma unroll
-    for (int c = 7; c >= 0; c--) {
-        const float t0 = fmaxf(mn[c], __fmaf_rn(n[c], r.inv[2], -r.near[2]));
-        const float t1 = fminf(mx[c], __fmaf_rn(f[c], r.inv[2], -r.far[2]));
-        m = __funnelshift_l(__float_as_uint(t1 - t0), m, 1);
+    for (int c = 3; c >= 0; c--) {
+        float a, b, t0, t1;
+        unpack2(fma2(n[c], r.inv[2], r.near[2]), a, b);
+        t0 = fmaxf(mn[2 * c], a);
+        t1 = fmaxf(mn[2 * c + 1], b);
+        unpack2(fma2(f[c], r.inv[2], r.far[2]), a, b);
+        m = __funnelshift_l(__float_as_uint(fminf(mx[2 * c + 1], b) - t1), m, 1);
+        m = __funnelshift_l(__float_as_uint(fminf(mx[2 * c], a) - t0), m, 1);
     }
     m = ~m & 0xFFu;
     if (order & 1) m = ((m & 0x55u) << 1) | ((m >> 1) & 0x55u);
