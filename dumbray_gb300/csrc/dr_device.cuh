@@ -131,6 +131,35 @@ __device__ __forceinline__ bool slab_hit(float lx, float ly, float lz, float hx,
     return mn != FLT_MAX;
 }
 
+// Two floats in one register pair, and operations on both (one issue slot on sm_100 and later), each
+// rounded as its scalar counterpart.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// xdot of two pairs of vectors
+__device__ __forceinline__ f32x2 xdot2(const f32x2 (&a)[3], const f32x2 (&b)[3]) {
+    return add2(add2(mul2(a[0], b[0]), mul2(a[1], b[1])), mul2(a[2], b[2]));
+}
+
 // One edge condition of Triangle::containsVertex (Triangle.impl.h:292-302), every operation exactly
 // rounded: rn(rn(X / rn(sqrt(P))) + S) >= rn(Y / rn(sqrt(Q))), X = e.px, P = px.px, Y = -(e.f), Q = f.f.
 // The right side depends on the triangle alone (edge_limit).
@@ -149,58 +178,72 @@ static __device__ __noinline__ bool contains_vertex(f3 a, f3 b, f3 c, f3 p, floa
            edge_ok(xsub(a, c), xsub(p, c), limit_c);
 }
 
-// An edge condition with rsqrtf (documented max error 2 ulp): the fast left side differs from the
-// exactly rounded one by at most ~3 ulp, so a difference D outside the margin
-// M = 2^-19 (|L| + |R| + S) (about 16 ulp) has the sign of the exact difference.  Returns D - M in
-// `in` (positive: certainly inside) and D + M in `out` (negative: certainly outside); both fail for
-// NaN and infinities, which leaves the decision to contains_vertex.
-__device__ __forceinline__ void edge_fast(f3 e, f3 px, float P, float limit, bool &in, bool &out) {
-    const float L = __fadd_rn(__fmul_rn(xdot(e, px), rsqrtf(P)), kEdgeSlack);
-    const float D = __fsub_rn(L, limit);
-    const float M = 1.9073486328125e-06f * (fabsf(L) + fabsf(limit) + kEdgeSlack);
+// An edge condition with rsqrtf (documented max error 2 ulp), X = e.px, P = px.px: the fast left side
+// L = X rsqrt(P) + S differs from the exactly rounded one by at most ~3 ulp of |L| + S.  A difference
+// D = L - limit beyond M = 2^-18 (|limit| + S), which is at least 2^-19 (|L| + |limit| + S) or about 16
+// ulp there, has the sign of the exact difference.  `in` stays true while every edge is certainly inside,
+// `out` becomes true at one that is certainly outside; neither for NaN and infinities, which leaves the
+// decision to contains_vertex.
+__device__ __forceinline__ void edge_fast(float X, float P, float limit, bool &in, bool &out) {
+    const float D = __fmaf_rn(X, rsqrtf(P), kEdgeSlack) - limit;
+    const float M = __fmaf_rn(fabsf(limit), 3.9e-6f, 3.9e-6f * kEdgeSlack);
     in = in && D > M;
     out = out || D < -M;
 }
 
-// Leaf reference (64 bytes): floats 0-8 the vertices a, b, c; 9-11 the plane normal (b - a) x (c - a);
-// 12-14 the right sides of the three edge conditions; 15 the triangle id.  The last seven are what a
-// test would otherwise compute again for every ray, with the same rounding.
+// Leaf reference (64 bytes), floats a.x b.x a.y b.y a.z b.z c.x c.y | c.z, the plane normal
+// (b - a) x (c - a), the right sides of the three edge conditions, the triangle id.  The normal and the
+// right sides are what a test would otherwise compute again for every ray, with the same rounding;
+// corners a and b lie side by side for the paired arithmetic.
 constexpr int kLeafTriF4 = 4;
 __device__ __forceinline__ int leaf_tri_id(const float4 *leaf_tris, int pos) {
     return __float_as_int(__ldg(leaf_tris + (size_t)pos * kLeafTriF4 + 3).w);
 }
-__device__ __forceinline__ void ldg8(const void *p, float *v) {
-    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-        : "l"(p));
+__device__ __forceinline__ void ldg8(const void *p, f32x2 *v) {
+    asm("ld.global.nc.v4.b64 {%0,%1,%2,%3}, [%4];" : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(p));
 }
 
 // Triangle::cast (Triangle.impl.h:334-348) of leaf reference `pos`, with the caller's validator check
 // (castInLeaf, Octree.impl.cuh:596-603) moved ahead of the containment test: the ignored triangle
 // cannot change the leaf's result.  The three edges are tested together: among the 32 tests of a
-// window some lane nearly always needs the last one.
+// window some lane nearly always needs the last one.  Differences are taken corner - p: the signs of
+// both factors of P and of X cancel or are undone exactly.
 __device__ __forceinline__ bool tri_cast(const float4 *leaf_tris, int pos, f3 o, f3 d, bool clip, int ignore, float &dist) {
-    const float4 *q = leaf_tris + (size_t)pos * kLeafTriF4;
-    float u[8], w[8];
-    ldg8(q, u);
-    ldg8(q + 2, w);
-    const f3 a = mkf3(u[0], u[1], u[2]), b = mkf3(u[3], u[4], u[5]), c = mkf3(u[6], u[7], w[0]), n = mkf3(w[1], w[2], w[3]);
+    const float4 *r = leaf_tris + (size_t)pos * kLeafTriF4;
+    f32x2 u[4], w[4];
+    ldg8(r, u);
+    ldg8(r + 2, w);
+    f3 a, b, c, n;
+    float limit_a, limit_b, limit_c, id;
+    unpack2(u[0], a.x, b.x);
+    unpack2(u[1], a.y, b.y);
+    unpack2(u[2], a.z, b.z);
+    unpack2(u[3], c.x, c.y);
+    unpack2(w[0], c.z, n.x);
+    unpack2(w[1], n.y, n.z);
+    unpack2(w[2], limit_a, limit_b);
+    unpack2(w[3], limit_c, id);
     const float dp = xdot(xsub(a, o), n);
     const float dirp = xdot(d, n);
     if ((clip && dp < -kEps) || __fmul_rn(dp, dirp) <= 0.0f) return false;
     dist = __fdiv_rn(dp, dirp);
-    if (!(dist < FLT_MAX) || __float_as_int(w[7]) == ignore) return false;
+    if (!(dist < FLT_MAX) || __float_as_int(id) == ignore) return false;
     const f3 p = xadd(o, xmul(d, dist));
-    const f3 pa = xsub(p, a), pb = xsub(p, b), pc = xsub(p, c);
-    const float Pa = xdot(pa, pa), Pb = xdot(pb, pb), Pc = xdot(pc, pc);
-    bool in = fminf(fminf(Pa, Pb), Pc) > 0.0f, out = false;   // on a vertex: the exact test decides
-    const bool vertex = !in;
-    edge_fast(xsub(b, a), pa, Pa, w[4], in, out);
-    edge_fast(xsub(c, b), pb, Pb, w[5], in, out);
-    edge_fast(xsub(a, c), pc, Pc, w[6], in, out);
+    const f32x2 q[3] = {add2(u[0], pack2(-p.x, -p.x)), add2(u[1], pack2(-p.y, -p.y)), add2(u[2], pack2(-p.z, -p.z))};
+    const f3 qc = xsub(c, p), ab = xsub(b, a), bc = xsub(c, b), ca = xsub(a, c);
+    const f32x2 e[3] = {pack2(ab.x, bc.x), pack2(ab.y, bc.y), pack2(ab.z, bc.z)};
+    float Xa, Xb, Pa, Pb;
+    unpack2(xdot2(e, q), Xa, Xb);
+    unpack2(xdot2(q, q), Pa, Pb);
+    const float Xc = xdot(ca, qc), Pc = xdot(qc, qc);
+    const bool vertex = !(fminf(fminf(Pa, Pb), Pc) > 0.0f);   // on a vertex: the exact test decides
+    bool in = !vertex, out = false;
+    edge_fast(-Xa, Pa, limit_a, in, out);
+    edge_fast(-Xb, Pb, limit_b, in, out);
+    edge_fast(-Xc, Pc, limit_c, in, out);
     if (in) return true;
     if (out && !vertex) return false;
-    return contains_vertex(a, b, c, p, w[4], w[5], w[6]);
+    return contains_vertex(a, b, c, p, limit_a, limit_b, limit_c);
 }
 
 struct Hit {
@@ -294,20 +337,6 @@ constexpr int kRecordF4 = 16;
 constexpr float kRecordPad = 1.0f / 524288.0f;
 constexpr float kRaySlack = 1.0f / 1048576.0f;
 
-// Two floats in one register pair, and a fused multiply-add of both (one issue slot on sm_100 and later).
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-    f32x2 v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-    return v;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-
 // What record_mask needs of a ray: 1 / d and the negated offsets of the near and far planes, each twice
 // in a pair.
 struct RaySlopes {
@@ -343,10 +372,6 @@ __device__ __forceinline__ RaySlopes ray_slopes(f3 o, f3 d, float reach) {
 __device__ __forceinline__ bool never_hits(f3 o, f3 d) {
     const float z = (o.x - o.x) + (o.y - o.y) + (o.z - o.z) + (d.x - d.x) + (d.y - d.y) + (d.z - d.z);
     return z != 0.0f || z != z || (d.x == 0.0f && d.y == 0.0f && d.z == 0.0f);
-}
-
-__device__ __forceinline__ void ldg8(const char *p, f32x2 *v) {
-    asm("ld.global.nc.v4.b64 {%0,%1,%2,%3}, [%4];" : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(p));
 }
 
 // Children of group `g` that the ray may enter, bit k = child (order ^ k), and the group's word 48.

@@ -148,14 +148,14 @@ struct BatchSource {
     int *hit_tri, *nbox, *ntri;
     float *hit_t;
     int n, chunk;
-    long long at;         // the warp's next chunk
+    unsigned at;          // the warp's next chunk
     bool cull;
     const Scene *scene0;  // unused: single-scene source
     __device__ __forceinline__ bool next(int &b, int &e) {
-        if (at >= n) return false;
+        if (at >= (unsigned)n) return false;
         b = (int)at;
-        e = min(b + chunk, n);
-        at += (long long)grid_warps() * chunk;
+        e = n - b > chunk ? b + chunk : n;
+        at += (unsigned)(grid_warps() * chunk);   // less than 2^31 + 2^18
         return true;
     }
     __device__ __forceinline__ bool load(int i, f3 &ro, f3 &rd, int &ign, int &job) {
@@ -168,7 +168,7 @@ struct BatchSource {
     __device__ __forceinline__ int job(int) { return 0; }
     // single-scene source: never asked for a per-job scene (MULTI = false)
     __device__ __forceinline__ const Scene &scene(int) { return *scene0; }
-    __device__ __forceinline__ bool clip(int) { return cull; }
+    __device__ __forceinline__ bool clip() { return cull; }
     __device__ __forceinline__ bool store(int i, const Hit &h, int nb, int nt) {
         hit_tri[i] = h.tri;
         hit_t[i] = h.tri >= 0 ? h.t : FLT_MAX;
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(kCastThreads, cast_blocks_per_sm(COUNT))
     typename StackOf<COUNT>::type stack[kStack];
     __shared__ WarpSlots slots[kCastThreads / 32];
     const int width = warp_width(n, grid_warps());
-    const long long warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const unsigned warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     BatchSource src{o, d, ignore, hit_tri, COUNT ? nbox : nullptr, COUNT ? ntri : nullptr, hit_t, n, width, warp * width, clip != 0, &S};
     trace_persistent<COUNT, false>(S, src, stack, slots[threadIdx.x >> 5], width, steps_per_round(S.front_only != 0));
 }
@@ -402,10 +402,7 @@ struct TraceSource {
     }
     __device__ __forceinline__ int job(int i) { return Q.p3[i].w; }
     __device__ __forceinline__ const Scene &scene(int job) { return job_of<MULTI>(*A, job).S; }
-    __device__ __forceinline__ bool clip(int job) {
-        const Item &I = job_of<MULTI>(*A, job);
-        return I.mode == DR_MODE_REFERENCE && I.clip != 0;
-    }
+    __device__ __forceinline__ bool clip() { return A->inl.mode == DR_MODE_REFERENCE && A->inl.clip != 0; }
     __device__ __forceinline__ bool store(int i, const Hit &h, int b_, int t_) {
         hits[i] = make_float2(__int_as_float(h.tri), h.t);
         rays++;
@@ -627,7 +624,7 @@ struct RefPhotonSource {
     }
     __device__ __forceinline__ int job(int i) { return __float_as_int(sq.s4[i].w); }
     __device__ __forceinline__ const Scene &scene(int job) { return job_of<MULTI>(*A, job).S; }
-    __device__ __forceinline__ bool clip(int job) { return job_of<MULTI>(*A, job).clip != 0; }
+    __device__ __forceinline__ bool clip() { return A->inl.clip != 0; }
     __device__ __forceinline__ bool store(int i, const Hit &h, int b_, int t_) {
         rays++;
         nb += b_;
@@ -710,7 +707,7 @@ struct RefPhotonChainSource {
     }
     __device__ __forceinline__ int job(int i) { return __float_as_int(sq.s4[kept ? kept[i] : i].w); }
     __device__ __forceinline__ const Scene &scene(int job) { return job_of<MULTI>(*A, job).S; }
-    __device__ __forceinline__ bool clip(int job) { return job_of<MULTI>(*A, job).clip != 0; }
+    __device__ __forceinline__ bool clip() { return A->inl.clip != 0; }
     __device__ __forceinline__ bool store(int i, const Hit &h, int b_, int t_) {
         rays++;
         nb += b_;
@@ -989,7 +986,7 @@ struct ShadowPhysSource {
     }
     __device__ __forceinline__ int job(int i) { return __float_as_int(sq.s4[i].w); }
     __device__ __forceinline__ const Scene &scene(int job) { return job_of<MULTI>(*A, job).S; }
-    __device__ __forceinline__ bool clip(int) { return false; }
+    __device__ __forceinline__ bool clip() { return false; }
     __device__ __forceinline__ bool store(int i, const Hit &h, int b_, int t_) {
         int light_tri = __float_as_int(sq.s1[i].w);
         bool vis = (h.tri < 0) || (h.tri == light_tri) || !(h.t < 0.999f);
@@ -1152,8 +1149,8 @@ __global__ void k_leaf_tris(float4 *dst, const int *refs, const float4 *tris, lo
         const f3 ab = xsub(t.b, t.a), bc = xsub(t.c, t.b), ca = xsub(t.a, t.c);
         const f3 n = xcross(ab, xsub(t.c, t.a));
         float4 *q = dst + r * kLeafTriF4;
-        q[0] = make_float4(t.a.x, t.a.y, t.a.z, t.b.x);
-        q[1] = make_float4(t.b.y, t.b.z, t.c.x, t.c.y);
+        q[0] = make_float4(t.a.x, t.b.x, t.a.y, t.b.y);
+        q[1] = make_float4(t.a.z, t.b.z, t.c.x, t.c.y);
         q[2] = make_float4(t.c.z, n.x, n.y, n.z);
         q[3] = make_float4(edge_limit(ab, ca), edge_limit(bc, ab), edge_limit(ca, bc), __int_as_float(id));
     }

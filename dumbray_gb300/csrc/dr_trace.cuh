@@ -152,7 +152,7 @@ __device__ __forceinline__ int warp_width(int n, int warps) { return max(1, min(
 //   bool load(int i, f3 &o, f3 &d, int &ignore, int &job)   false: entry i needs no cast (done)
 //   int job(int i)                            the job of entry i
 //   const Scene &scene(int job)               the scene of a job (MULTI only)
-//   bool clip(int job)                        backface culling of a job (MULTI = false: job 0 for all)
+//   bool clip()                               backface culling (of the first job: the same for all)
 //   bool store(int i, const Hit &h, int nbox, int ntri)   true: ray i was rewritten (load() now
 //                                             gives its next cast) and the lane traces it at once
 //   static constexpr float kOccludeBelow      > 0: visibility-only rays (any hit nearer than this
@@ -179,7 +179,7 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ty
     bool drained = false;
     int cur_i = -1;
     int mode = kIdle;
-    const bool clip = src.clip(0);
+    const bool clip = src.clip();
     const bool front = !COUNT || S.front_only != 0;   // uniform: one scene, or one arena of a batch
     // group-test planes of a counting traversal: the reference's boxes on reference-padding scenes
     // (their counts are the reference's), the refitted ones elsewhere
