@@ -76,48 +76,70 @@ __global__ void k_centres(const float *xyz, const int *refs, const int *owner, c
     centre[3 * (size_t)r + 2] = c.z;
 }
 
-// One warp per node: the lanes load 32 centres at a time and every lane adds them in list order
-// (broadcast one by one), so the float sum has the host builder's order.
-__global__ void k_split_points(const float *centre, const int *off, const float *box, int nl, int depth, int max_depth,
-                               int split_n, float E, float *sub) {
+// One warp per node: the lanes stage kStage centres at a time in shared memory, axis by axis, and lanes
+// 0-2 add one axis each in list order, so the float sum has the host builder's order.  The chain of
+// dependent additions is what a large node costs (4 cycles each, three shuffles and 58 cycles a
+// reference when every lane added broadcast values); the next stage's loads are issued before it.
+constexpr int kStage = 128, kStageWarps = 4;
+__global__ void __launch_bounds__(32 * kStageWarps) k_split_points(const float *centre, const int *off, const float *box, int nl, int depth,
+                                                                   int max_depth, int split_n, float E, float *sub) {
+    __shared__ __align__(16) float stage[kStageWarps][3][kStage];
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (k >= nl || !splittable(off, k, depth, max_depth, split_n)) return;
+    float (&st)[3][kStage] = stage[threadIdx.x >> 5];
     const int rb = off[k], re = off[k + 1];
-    P3 c = mk(0, 0, 0);
-    for (int base = rb; base < re; base += 32) {
-        const int r = base + lane;
-        float x = 0.0f, y = 0.0f, z = 0.0f;
-        if (r < re) {
-            x = centre[3 * (size_t)r];
-            y = centre[3 * (size_t)r + 1];
-            z = centre[3 * (size_t)r + 2];
+    constexpr int kLoads = 3 * kStage / 32;
+    float v[kLoads];
+    auto load = [&](int base) {
+        const int m = 3 * min(kStage, re - base);
+        const float *c = centre + 3 * (size_t)base;
+#pragma unroll
+        for (int j = 0; j < kLoads; j++) v[j] = 32 * j + lane < m ? c[32 * j + lane] : 0.0f;
+    };
+    load(rb);
+    float sum = 0.0f;
+    for (int base = rb; base < re; base += kStage) {
+#pragma unroll
+        for (int j = 0; j < kLoads; j++) st[(32 * j + lane) % 3][(32 * j + lane) / 3] = v[j];
+        __syncwarp();
+        if (base + kStage < re) load(base + kStage);
+        if (lane < 3) {
+            const int m = min(kStage, re - base);
+            int j = 0;
+            for (; j + 4 <= m; j += 4) {
+                const float4 q = *reinterpret_cast<const float4 *>(&st[lane][j]);
+                sum = (((sum + q.x) + q.y) + q.z) + q.w;
+            }
+            for (; j < m; j++) sum += st[lane][j];
         }
-        const int m = min(32, re - base);
-        for (int j = 0; j < m; j++)
-            c = add(c, mk(__shfl_sync(0xFFFFFFFFu, x, j), __shfl_sync(0xFFFFFFFFu, y, j), __shfl_sync(0xFFFFFFFFu, z, j)));
+        __syncwarp();
     }
+    const P3 c = divs(mk(__shfl_sync(0xFFFFFFFFu, sum, 0), __shfl_sync(0xFFFFFFFFu, sum, 1), __shfl_sync(0xFFFFFFFFu, sum, 2)),
+                      (float)(re - rb));
     if (lane != 0) return;
-    c = divs(c, (float)(re - rb));
     Bx o[8];
     octants(load_box(box, k), c, o, E);
     for (int i = 0; i < 8; i++) store_box(sub, 8 * k + i, o[i]);
 }
 
+// Same call, scenes of the displaced icosphere, physical padding, split 4: with these three kernels
+// (sums, masks, lists) 82k triangles 22.2 -> 18.6 ms, 1.31M triangles 352 -> 297 ms.
+//
+// Octant overlap of every reference: a thread per (reference, octant), the mask byte from a ballot.
+// (One thread per reference took its eight tests one after another, each as long as the longest of the
+// warp's.)
 __global__ void k_masks(const float *xyz, const int *refs, const int *owner, const int *off, const float *sub, int nr, int depth,
                         int max_depth, int split_n, unsigned char *mask) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= nr) return;
-    const int k = owner[r];
-    if (!splittable(off, k, depth, max_depth, split_n)) {
-        mask[r] = 0;
-        return;
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const int r = (int)(t >> 3), i = (int)(t & 7);
+    bool hit = false;
+    if (r < nr) {
+        const int k = owner[r];
+        if (splittable(off, k, depth, max_depth, split_n)) hit = overlaps(load_box(sub, 8 * k + i), load_tri(xyz, refs[r]));
     }
-    const T3 t = load_tri(xyz, refs[r]);
-    unsigned m = 0;
-    for (int i = 0; i < 8; i++)
-        if (overlaps(load_box(sub, 8 * k + i), t)) m |= 1u << i;
-    mask[r] = (unsigned char)m;
+    const unsigned bal = __ballot_sync(0xFFFFFFFFu, hit);
+    if (r < nr && i == 0) mask[r] = (unsigned char)(bal >> (threadIdx.x & 24));
 }
 
 // splittingMakesSence (Octree.impl.cuh:437-475): one warp per node.
@@ -187,26 +209,78 @@ __global__ void k_leaf_boxes(const float *bounds, const int *off, const float *b
     if (lane == 0) store_box(lbox, k, shrink(b, lo, hi, E));
 }
 
-// Children's reference lists (Octree.impl.cuh:392-404): one thread per split node.
-__global__ void k_scatter(const int *refs, const unsigned char *mask, const int *off, const int *first_child, const int *next_off,
-                          int nl, int *next_refs) {
-    const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (k >= nl || first_child[k] < 0) return;
+// Children's reference lists (Octree.impl.cuh:392-404), in list order: a reference's position in an
+// octant's list is the count of earlier references that also overlap it.  A warp per split node, 32
+// references at a time by ballots; nodes of more than kBlockRefs references go to the whole block
+// afterwards, 4 references a thread: counts per octant as bytes of a 64-bit word, scanned over the warp
+// by shuffles and over the block in shared memory.
+constexpr int kScatterWarps = 8, kBlockRefs = 2048, kPerThread = 4;
+__global__ void __launch_bounds__(32 * kScatterWarps) k_scatter(const int *refs, const unsigned char *mask, const int *off, const int *first_child,
+                                                                const int *next_off, int nl, int *next_refs) {
+    __shared__ int totals[kScatterWarps][8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
-    int w[8];
-    for (int i = 0; i < 8; i++) w[i] = next_off[first_child[k] + i];
-    // chunks of 32 references in list order; within a chunk, a lane's position among the chunk's
-    // references overlapping octant i is the count of lower lanes that also do
-    for (int base = off[k]; base < off[k + 1]; base += 32) {
-        const int r = base + lane;
-        const bool in = r < off[k + 1];
-        const unsigned m = in ? mask[r] : 0u;
-        const int id = in ? refs[r] : 0;
-        for (int i = 0; i < 8; i++) {
-            const unsigned bal = __ballot_sync(0xFFFFFFFFu, (m >> i) & 1u);
-            if ((m >> i) & 1u) next_refs[w[i] + __popc(bal & lt)] = id;
-            w[i] += __popc(bal);
+    const int k0 = blockIdx.x * kScatterWarps;
+    const int k = k0 + warp;
+    if (k < nl && first_child[k] >= 0 && off[k + 1] - off[k] <= kBlockRefs) {
+        int w[8];
+        for (int i = 0; i < 8; i++) w[i] = next_off[first_child[k] + i];
+        for (int base = off[k]; base < off[k + 1]; base += 32) {
+            const int r = base + lane;
+            const bool in = r < off[k + 1];
+            const unsigned m = in ? mask[r] : 0u;
+            const int id = in ? refs[r] : 0;
+            for (int i = 0; i < 8; i++) {
+                const unsigned bal = __ballot_sync(0xFFFFFFFFu, (m >> i) & 1u);
+                if ((m >> i) & 1u) next_refs[w[i] + __popc(bal & lt)] = id;
+                w[i] += __popc(bal);
+            }
+        }
+    }
+    for (int j = k0; j < min(k0 + kScatterWarps, nl); j++) {
+        const int rb = off[j], re = off[j + 1];
+        if (first_child[j] < 0 || re - rb <= kBlockRefs) continue;   // the same for the whole block
+        int w[8];
+        for (int i = 0; i < 8; i++) w[i] = next_off[first_child[j] + i];
+        unsigned char m[kPerThread];
+        int id[kPerThread];
+        auto load = [&](int base) {
+            for (int q = 0; q < kPerThread; q++) {
+                const int r = base + kPerThread * (int)threadIdx.x + q;
+                m[q] = r < re ? mask[r] : 0;
+                id[q] = r < re ? refs[r] : 0;
+            }
+        };
+        load(rb);
+        for (int base = rb; base < re; base += 32 * kScatterWarps * kPerThread) {
+            // bit i of a mask -> byte i of a word: at most 4 a thread, 128 a warp
+            unsigned long long mine = 0;
+            for (int q = 0; q < kPerThread; q++)
+                for (int i = 0; i < 8; i++) mine += (unsigned long long)((m[q] >> i) & 1u) << (8 * i);
+            unsigned long long incl = mine;
+            for (int s = 1; s < 32; s <<= 1) {
+                const unsigned long long v = __shfl_up_sync(0xFFFFFFFFu, incl, s);
+                if (lane >= s) incl += v;
+            }
+            if (lane == 31)
+                for (int i = 0; i < 8; i++) totals[warp][i] = (int)((incl >> (8 * i)) & 0xFF);
+            __syncthreads();
+            const unsigned long long excl = incl - mine;
+            int at[8];
+            for (int i = 0; i < 8; i++) {
+                int before = 0, all = 0;
+                for (int v = 0; v < kScatterWarps; v++) {
+                    if (v < warp) before += totals[v][i];
+                    all += totals[v][i];
+                }
+                at[i] = w[i] + before + (int)((excl >> (8 * i)) & 0xFF);
+                w[i] += all;
+            }
+            for (int q = 0; q < kPerThread; q++)
+                for (int i = 0; i < 8; i++)
+                    if ((m[q] >> i) & 1u) next_refs[at[i]++] = id[q];
+            load(base + 32 * kScatterWarps * kPerThread);
+            __syncthreads();
         }
     }
 }
@@ -331,8 +405,8 @@ bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, Flat
             k_owner<<<blocks(nr, 256), 256>>>(d_off, nl, nr, d_owner);
             k_centres<<<blocks(nr, 128), 128>>>(d_xyz, d_refs, d_owner, d_off, d_box, nr, depth, max_depth, split_n, d_centre);
         }
-        k_split_points<<<blocks(32LL * nl, 256), 256>>>(d_centre, d_off, d_box, nl, depth, max_depth, split_n, E, d_sub);
-        if (nr > 0) k_masks<<<blocks(nr, 128), 128>>>(d_xyz, d_refs, d_owner, d_off, d_sub, nr, depth, max_depth, split_n, d_mask);
+        k_split_points<<<blocks(nl, kStageWarps), 32 * kStageWarps>>>(d_centre, d_off, d_box, nl, depth, max_depth, split_n, E, d_sub);
+        if (nr > 0) k_masks<<<blocks(8LL * nr, 256), 256>>>(d_xyz, d_refs, d_owner, d_off, d_sub, nr, depth, max_depth, split_n, d_mask);
         k_decide<<<blocks(32LL * nl, 256), 256>>>(d_mask, d_off, nl, depth, max_depth, split_n, d_occ, d_split);
         if (nr > 0) k_leaf_bounds<<<blocks(nr, 128), 128>>>(d_xyz, d_refs, d_owner, d_box, d_split, nr, d_bounds);
         k_leaf_boxes<<<blocks(32LL * nl, 256), 256>>>(d_bounds, d_off, d_box, d_split, nl, E, d_lbox);
@@ -406,7 +480,7 @@ bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, Flat
             if (!d_fc || !d_noff || !d_next) { err = "device allocation failed"; return false; }
             cudaMemcpy(d_fc, h_fc.data(), 4 * (size_t)nl, cudaMemcpyHostToDevice);
             cudaMemcpy(d_noff, h_noff.data(), 4 * (size_t)(nn + 1), cudaMemcpyHostToDevice);
-            k_scatter<<<blocks(32LL * nl, 256), 256>>>(d_refs, d_mask, d_off, d_fc, d_noff, nl, d_next);
+            k_scatter<<<blocks(nl, kScatterWarps), 32 * kScatterWarps>>>(d_refs, d_mask, d_off, d_fc, d_noff, nl, d_next);
             e = cudaGetLastError();
             if (e == cudaSuccess) e = cudaDeviceSynchronize();
             if (e != cudaSuccess) {
