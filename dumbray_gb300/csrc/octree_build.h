@@ -39,8 +39,7 @@ struct FlatOctree {
 // xyz: float[n][3][3].  Returns false on invalid input.
 bool build_octree(const float *xyz, int64_t n, const BuildOptions &opt, FlatOctree &out);
 
-// The same build on the current CUDA device (octree_gpu.cu): per-reference clipping and per-node
-// passes on the GPU, level bookkeeping on the host; bit-identical output.  err: reason on failure.
+// The same build on the current CUDA device (octree_gpu.cu); bit-identical output.  err: reason on failure.
 bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, FlatOctree &out, std::string &err);
 
 }  // namespace drb

@@ -5,22 +5,24 @@
 //   (1) owner of every reference (binary search over the level's reference ranges),
 //   (2) the clipped centre of every reference of a splittable node (parallel over references),
 //   (3) the split point of every splittable node: the float sum of its references' centres in list
-//       order (a warp per node loads, every lane adds in list order: the order of a float sum is part
-//       of the result) and its octants,
+//       order (a warp per node loads, a lane per axis adds: the order of a float sum is part of the
+//       result) and its octants,
 //   (4) the octant overlap mask of every reference (parallel),
 //   (5) per node the octant occupancy and the split decision (a warp per node; integer sums),
 //   (6) the clipped bounds of every reference of a leaf (parallel) and each leaf's box: min / max in
 //       list order from the node box, then the padded shrink (a warp per leaf),
-//   (7) the children's reference lists: for every split node its references copied to the lists of
-//       the octants they overlap, in list order (a warp per node: ballots and prefix counts).
-// The host keeps the level bookkeeping (which nodes split, where children and leaf lists go), which
-// is the host builder's own step 6, and the final bottom-up box reduce.  All geometry comes from
-// octree_geom.h; nvcc compiles it with -fmad=false and IEEE division / square root, the host builder
-// with -ffp-contract=off, so both perform the same single-precision operations.
+//   (7) prefix sums over the level's nodes of their split flags, leaf references and child references:
+//       where each split node's children and each leaf's list go (breadth-first order),
+//   (8) the next level's nodes and, for every split node, its references copied to the lists of the
+//       octants they overlap, in list order (a warp per node, the block for large ones).
+// After the last level inner boxes shrink to their children's, level by level from the deepest.  The
+// host reads three totals a level (sizes of the next level's arrays) and the finished tree.  All geometry
+// comes from octree_geom.h; nvcc compiles it with -fmad=false and IEEE division / square root, the host
+// builder with -ffp-contract=off, so both perform the same single-precision operations.
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -49,6 +51,11 @@ __device__ __forceinline__ void store_box(float *b, int k, const Bx &x) {
 }
 __device__ __forceinline__ bool splittable(const int *off, int k, int depth, int max_depth, int split_n) {
     return depth < max_depth && (off[k + 1] - off[k]) >= split_n;
+}
+
+__global__ void k_iota(int *v, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) v[i] = i;
 }
 
 __global__ void k_owner(const int *off, int nl, int nr, int *owner) {
@@ -142,9 +149,19 @@ __global__ void k_masks(const float *xyz, const int *refs, const int *owner, con
     if (r < nr && i == 0) mask[r] = (unsigned char)(bal >> (threadIdx.x & 24));
 }
 
+// What a node adds to the level's prefix sums.  (Splits, lists and boxes of a level used to go to the host
+// for this bookkeeping: 82k triangles 17.3 -> 12.6 ms, 1.31M triangles 291 -> 169 ms a scene, same call.)
+struct Sums {
+    int splits, leaf_refs;
+    long long child_refs;
+};
+__host__ __device__ __forceinline__ Sums operator+(Sums a, Sums b) {
+    return Sums{a.splits + b.splits, a.leaf_refs + b.leaf_refs, a.child_refs + b.child_refs};
+}
+
 // splittingMakesSence (Octree.impl.cuh:437-475): one warp per node.
 __global__ void k_decide(const unsigned char *mask, const int *off, int nl, int depth, int max_depth, int split_n, int *occ,
-                         int *does_split) {
+                         int *does_split, Sums *sums) {
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (k >= nl) return;
@@ -170,7 +187,126 @@ __global__ void k_decide(const unsigned char *mask, const int *off, int nl, int 
         ok = (full < 1) && (load < fminf(((float)cnt) / ((float)split_n), 6.0f));
     }
     does_split[k] = ok ? 1 : 0;
-    for (int i = 0; i < 8; i++) occ[8 * k + i] = c[i];
+    long long all = 0;
+    for (int i = 0; i < 8; i++) {
+        occ[8 * k + i] = c[i];
+        all += c[i];
+    }
+    sums[k] = ok ? Sums{1, 0, all} : Sums{0, off[k + 1] - off[k], 0};
+}
+
+// Exclusive prefix sums in place: chunks of kScan nodes a block, the chunk totals by one block (the grand
+// total after the last).  The sum before node k is sums[k] + totals[k / kScan].
+constexpr int kScanThreads = 256, kScan = 4 * kScanThreads;
+__device__ __forceinline__ Sums block_scan(Sums v, Sums &total) {   // exclusive, over the block's threads
+    __shared__ Sums warps[kScanThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Sums x = v;
+    for (int s = 1; s < 32; s <<= 1) {
+        const Sums y{__shfl_up_sync(0xFFFFFFFFu, x.splits, s), __shfl_up_sync(0xFFFFFFFFu, x.leaf_refs, s),
+                     __shfl_up_sync(0xFFFFFFFFu, x.child_refs, s)};
+        if (lane >= s) x = x + y;
+    }
+    __syncthreads();   // a caller's previous scan is read
+    if (lane == 31) warps[warp] = x;
+    __syncthreads();
+    Sums before{0, 0, 0};
+    total = before;
+    for (int w = 0; w < kScanThreads / 32; w++) {
+        if (w == warp) before = total;
+        total = total + warps[w];
+    }
+    return Sums{before.splits + x.splits - v.splits, before.leaf_refs + x.leaf_refs - v.leaf_refs,
+                before.child_refs + x.child_refs - v.child_refs};
+}
+__global__ void __launch_bounds__(kScanThreads) k_scan_chunks(Sums *sums, int n, Sums *totals) {
+    const long long first = (long long)blockIdx.x * kScan + 4 * threadIdx.x;
+    Sums v[4], all{0, 0, 0}, total;
+    for (int q = 0; q < 4; q++) {
+        v[q] = first + q < n ? sums[first + q] : Sums{0, 0, 0};
+        all = all + v[q];
+    }
+    Sums at = block_scan(all, total);
+    for (int q = 0; q < 4; q++) {
+        if (first + q < n) sums[first + q] = at;
+        at = at + v[q];
+    }
+    if (threadIdx.x == 0) totals[blockIdx.x] = total;
+}
+__global__ void __launch_bounds__(kScanThreads) k_scan_totals(Sums *totals, int m) {
+    Sums carry{0, 0, 0};
+    for (int base = 0; base < m; base += kScanThreads) {
+        const int i = base + (int)threadIdx.x;
+        Sums total;
+        const Sums at = block_scan(i < m ? totals[i] : Sums{0, 0, 0}, total);
+        if (i < m) totals[i] = carry + at;
+        carry = carry + total;
+    }
+    if (threadIdx.x == 0) totals[m] = carry;
+}
+__device__ __forceinline__ Sums sums_before(const Sums *sums, const Sums *totals, int k) { return sums[k] + totals[k / kScan]; }
+
+// The level's finished nodes and the next level's: one thread per node.  A split node's children start at
+// 8 x the split nodes before it, in the next level and (plus next_base) in the tree; a leaf takes its
+// shrunk box and its place in the tree's reference list.
+__global__ void k_emit(const Sums *sums, const Sums *totals, const int *off, const int *does_split, const int *occ, const float *sub,
+                       const float *lbox, int nl, long long leaf_base, int next_base, float *box, int *child, int *first_child,
+                       long long *leaf_first, int *leaf_count, int *next_off, float *next_box) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nl) return;
+    const Sums at = sums_before(sums, totals, k);
+    if (!does_split[k]) {
+        store_box(box, k, load_box(lbox, k));
+        child[k] = -1;
+        first_child[k] = -1;
+        leaf_first[k] = leaf_base + at.leaf_refs;
+        leaf_count[k] = off[k + 1] - off[k];
+        return;
+    }
+    child[k] = next_base + 8 * at.splits;
+    first_child[k] = 8 * at.splits;
+    leaf_first[k] = 0;
+    leaf_count[k] = 0;
+    int r = (int)at.child_refs;
+    for (int i = 0; i < 8; i++) {
+        next_off[8 * at.splits + i] = r;
+        r += occ[8 * k + i];
+        store_box(next_box, 8 * at.splits + i, load_box(sub, 8 * k + i));
+    }
+    if (8LL * (at.splits + 1) == 8LL * totals[(nl + kScan - 1) / kScan].splits) next_off[8 * at.splits + 8] = r;   // the last one
+}
+
+// The leaves' references into the tree's list.
+__global__ void k_leaf_refs(const Sums *sums, const Sums *totals, const int *refs, const int *owner, const int *off, const int *does_split,
+                            int nr, int *out) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= nr) return;
+    const int k = owner[r];
+    if (!does_split[k]) out[sums_before(sums, totals, k).leaf_refs + r - off[k]] = refs[r];
+}
+
+// reduceNode(0, false) after the build: inner boxes shrink to the union of their children's; `child` less
+// `next_base` is the first child's place in the next level.
+__global__ void k_reduce(float *box, const int *child, int nl, int next_base, const float *next_box, float E) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nl || child[k] < 0) return;
+    const Bx b = load_box(box, k);
+    P3 lo = b.hi, hi = b.lo;
+    for (int c = 0; c < 8; c++) {
+        const Bx cb = load_box(next_box, child[k] - next_base + c);
+        lo = mk(fmin_(lo.x, cb.lo.x), fmin_(lo.y, cb.lo.y), fmin_(lo.z, cb.lo.z));
+        hi = mk(fmax_(hi.x, cb.hi.x), fmax_(hi.y, cb.hi.y), fmax_(hi.z, cb.hi.z));
+    }
+    store_box(box, k, shrink(b, lo, hi, E));
+}
+
+// A level's nodes into the finished arrays.
+__global__ void k_finish(const float *box, int nl, float *lo, float *hi) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= 3 * nl) return;
+    const int k = i / 3, a = i - 3 * k;
+    lo[i] = box[6 * (size_t)k + a];
+    hi[i] = box[6 * (size_t)k + 3 + a];
 }
 
 __global__ void k_leaf_bounds(const float *xyz, const int *refs, const int *owner, const float *box, const int *does_split,
@@ -302,11 +438,13 @@ struct DevBuf {
     T *get(size_t count) {
         const size_t need = std::max<size_t>(count, 1) * sizeof(T);
         if (need > bytes) {
+            // half as much again, so that the growing levels do not allocate each time
+            const size_t take = bytes ? need + need / 2 : need;
             cudaFree(p);
             p = nullptr;
             bytes = 0;
-            if (cudaMalloc(&p, need) != cudaSuccess) return nullptr;
-            bytes = need;
+            if (cudaMalloc(&p, take) != cudaSuccess) return nullptr;
+            bytes = take;
         }
         return (T *)p;
     }
@@ -342,51 +480,40 @@ bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, Flat
         }
     }
 
-    DevBuf b_xyz, b_refs, b_next, b_owner, b_centre, b_bounds, b_mask, b_off, b_noff, b_box, b_sub, b_occ, b_split, b_lbox, b_fc;
+    DevBuf b_xyz, b_refs, b_next, b_owner, b_centre, b_bounds, b_mask, b_off, b_noff, b_sub, b_occ, b_split, b_lbox, b_fc, b_sums, b_tot;
     float *d_xyz = b_xyz.get<float>(9 * (size_t)n);
     int *d_refs = b_refs.get<int>((size_t)n);
     if (!d_xyz || !d_refs) { err = "device allocation failed"; return false; }
     cudaMemcpy(d_xyz, xyz, 36 * (size_t)n, cudaMemcpyHostToDevice);
-    {
-        std::vector<int> ids((size_t)n);
-        for (int64_t i = 0; i < n; i++) ids[i] = (int)i;
-        cudaMemcpy(d_refs, ids.data(), 4 * (size_t)n, cudaMemcpyHostToDevice);
-    }
+    k_iota<<<blocks(n, 256), 256>>>(d_refs, (int)n);
 
-    struct LevelNode {
-        Bx box;
-        int rb, re;
-        int64_t global;
+    // what the tree keeps of every level
+    struct Level {
+        DevBuf box, child, first, count, leaf;
+        int nodes = 0, base = 0;     // base: the level's first node in the tree (the root has none)
+        long long leaf_base = 0;
+        int leaf_refs = 0;
     };
-    std::vector<LevelNode> level{{root, 0, (int)n, -1}};
-    std::vector<Bx> boxes;
-    std::vector<int32_t> child;
-    std::vector<int64_t> leaf_lo;
-    std::vector<int32_t> leaf_cnt;
-    std::vector<int32_t> &leaf_refs = out.leaf_refs;
-    Bx root_box = root;
-    int32_t root_child = -1;
-    int64_t root_leaf_lo = 0;
-    int32_t root_leaf_cnt = 0;
-    int max_seen = 0;
-    std::vector<int> h_off, h_split, h_occ, h_refs, h_fc, h_noff;
-    std::vector<float> h_box, h_sub, h_lbox;
-
-    for (int depth = 0; !level.empty(); depth++) {
-        max_seen = std::max(max_seen, depth);
-        const int nl = (int)level.size();
-        const int nr = level.back().re;
-        h_off.resize(nl + 1);
-        h_box.resize(6 * (size_t)nl);
-        for (int k = 0; k < nl; k++) {
-            h_off[k] = level[k].rb;
-            const Bx &b = level[k].box;
-            float *p = &h_box[6 * (size_t)k];
-            p[0] = b.lo.x; p[1] = b.lo.y; p[2] = b.lo.z; p[3] = b.hi.x; p[4] = b.hi.y; p[5] = b.hi.z;
-        }
-        h_off[nl] = nr;
-        int *d_off = b_off.get<int>(nl + 1);
-        float *d_box = b_box.get<float>(6 * (size_t)nl);
+    std::vector<std::unique_ptr<Level>> levels;
+    levels.push_back(std::make_unique<Level>());
+    levels[0]->nodes = 1;
+    {
+        const float b[6] = {root.lo.x, root.lo.y, root.lo.z, root.hi.x, root.hi.y, root.hi.z};
+        const int off[2] = {0, (int)n};
+        float *d_box = levels[0]->box.get<float>(6);
+        int *d_off = b_off.get<int>(2);
+        if (!d_box || !d_off) { err = "device allocation failed"; return false; }
+        cudaMemcpy(d_box, b, sizeof(b), cudaMemcpyHostToDevice);
+        cudaMemcpy(d_off, off, sizeof(off), cudaMemcpyHostToDevice);
+    }
+    int nr = (int)n, next_base = 0;
+    long long leaf_total = 0;
+    for (int depth = 0;; depth++) {
+        Level &lv = *levels[depth];
+        const int nl = lv.nodes;
+        const int chunks = (nl + kScan - 1) / kScan;
+        const int *d_off = (const int *)b_off.p;
+        float *d_box = (float *)lv.box.p;
         int *d_owner = b_owner.get<int>(nr);
         float *d_centre = b_centre.get<float>(3 * (size_t)nr);
         float *d_sub = b_sub.get<float>(48 * (size_t)nl);
@@ -395,142 +522,118 @@ bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, Flat
         int *d_split = b_split.get<int>(nl);
         float *d_bounds = b_bounds.get<float>(6 * (size_t)nr);
         float *d_lbox = b_lbox.get<float>(6 * (size_t)nl);
-        if (!d_off || !d_box || !d_owner || !d_centre || !d_sub || !d_mask || !d_occ || !d_split || !d_bounds || !d_lbox) {
+        Sums *d_sums = b_sums.get<Sums>(nl), *d_tot = b_tot.get<Sums>(chunks + 1);
+        int *d_fc = b_fc.get<int>(nl);
+        int *d_child = lv.child.get<int>(nl), *d_count = lv.count.get<int>(nl);
+        long long *d_first = lv.first.get<long long>(nl);
+        if (!d_owner || !d_centre || !d_sub || !d_mask || !d_occ || !d_split || !d_bounds || !d_lbox || !d_sums || !d_tot || !d_fc ||
+            !d_child || !d_count || !d_first) {
             err = "device allocation failed";
             return false;
         }
-        cudaMemcpy(d_off, h_off.data(), 4 * (size_t)(nl + 1), cudaMemcpyHostToDevice);
-        cudaMemcpy(d_box, h_box.data(), 24 * (size_t)nl, cudaMemcpyHostToDevice);
         if (nr > 0) {
             k_owner<<<blocks(nr, 256), 256>>>(d_off, nl, nr, d_owner);
             k_centres<<<blocks(nr, 128), 128>>>(d_xyz, d_refs, d_owner, d_off, d_box, nr, depth, max_depth, split_n, d_centre);
         }
         k_split_points<<<blocks(nl, kStageWarps), 32 * kStageWarps>>>(d_centre, d_off, d_box, nl, depth, max_depth, split_n, E, d_sub);
         if (nr > 0) k_masks<<<blocks(8LL * nr, 256), 256>>>(d_xyz, d_refs, d_owner, d_off, d_sub, nr, depth, max_depth, split_n, d_mask);
-        k_decide<<<blocks(32LL * nl, 256), 256>>>(d_mask, d_off, nl, depth, max_depth, split_n, d_occ, d_split);
+        k_decide<<<blocks(32LL * nl, 256), 256>>>(d_mask, d_off, nl, depth, max_depth, split_n, d_occ, d_split, d_sums);
         if (nr > 0) k_leaf_bounds<<<blocks(nr, 128), 128>>>(d_xyz, d_refs, d_owner, d_box, d_split, nr, d_bounds);
         k_leaf_boxes<<<blocks(32LL * nl, 256), 256>>>(d_bounds, d_off, d_box, d_split, nl, E, d_lbox);
+        k_scan_chunks<<<chunks, kScanThreads>>>(d_sums, nl, d_tot);
+        k_scan_totals<<<1, kScanThreads>>>(d_tot, chunks);
+        Sums total;
         cudaError_t e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaDeviceSynchronize();
+        if (e == cudaSuccess) e = cudaMemcpy(&total, d_tot + chunks, sizeof(Sums), cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) {
             err = std::string("device build: ") + cudaGetErrorString(e);
             return false;
         }
-        h_split.resize(nl);
-        h_occ.resize(8 * (size_t)nl);
-        h_sub.resize(48 * (size_t)nl);
-        h_lbox.resize(6 * (size_t)nl);
-        h_refs.resize(nr);
-        cudaMemcpy(h_split.data(), d_split, 4 * (size_t)nl, cudaMemcpyDeviceToHost);
-        cudaMemcpy(h_occ.data(), d_occ, 32 * (size_t)nl, cudaMemcpyDeviceToHost);
-        cudaMemcpy(h_sub.data(), d_sub, 192 * (size_t)nl, cudaMemcpyDeviceToHost);
-        cudaMemcpy(h_lbox.data(), d_lbox, 24 * (size_t)nl, cudaMemcpyDeviceToHost);
-        if (nr > 0) cudaMemcpy(h_refs.data(), d_refs, 4 * (size_t)nr, cudaMemcpyDeviceToHost);
-        auto hbox = [](const std::vector<float> &v, size_t k) {
-            const float *p = &v[6 * k];
-            return Bx{mk(p[0], p[1], p[2]), mk(p[3], p[4], p[5])};
-        };
-
-        // bookkeeping of the host builder's step 6
-        std::vector<LevelNode> next;
-        h_fc.assign(nl, -1);
-        int64_t next_refs = 0;
-        for (int k = 0; k < nl; k++) {
-            LevelNode &ln = level[k];
-            if (!h_split[k]) {
-                const int64_t lo = (int64_t)leaf_refs.size();
-                leaf_refs.insert(leaf_refs.end(), h_refs.begin() + ln.rb, h_refs.begin() + ln.re);
-                const int32_t cnt = ln.re - ln.rb;
-                const Bx lb = hbox(h_lbox, k);
-                if (ln.global < 0) { root_box = lb; root_leaf_lo = lo; root_leaf_cnt = cnt; }
-                else { boxes[ln.global] = lb; leaf_lo[ln.global] = lo; leaf_cnt[ln.global] = cnt; }
-                continue;
-            }
-            const int64_t first = (int64_t)boxes.size();
-            if (ln.global < 0) root_child = (int32_t)first;
-            else child[ln.global] = (int32_t)first;
-            h_fc[k] = (int)next.size();
-            for (int i = 0; i < 8; i++) {
-                const Bx sb = hbox(h_sub, 8 * (size_t)k + i);
-                boxes.push_back(sb);
-                child.push_back(-1);
-                leaf_lo.push_back(0);
-                leaf_cnt.push_back(0);
-                LevelNode c;
-                c.box = sb;
-                c.rb = (int)next_refs;
-                next_refs += h_occ[8 * (size_t)k + i];
-                c.re = (int)next_refs;
-                c.global = first + i;
-                next.push_back(c);
-            }
-        }
-        if (next_refs >= (int64_t(1) << 31)) {
+        if (total.child_refs >= (int64_t(1) << 31)) {
             err = "too many references in one level for the device build";
             return false;
         }
-        if (!next.empty()) {
-            const int nn = (int)next.size();
-            h_noff.resize(nn + 1);
-            for (int j = 0; j < nn; j++) h_noff[j] = next[j].rb;
-            h_noff[nn] = (int)next_refs;
-            int *d_fc = b_fc.get<int>(nl);
-            int *d_noff = b_noff.get<int>(nn + 1);
-            int *d_next = b_next.get<int>((size_t)next_refs);
-            if (!d_fc || !d_noff || !d_next) { err = "device allocation failed"; return false; }
-            cudaMemcpy(d_fc, h_fc.data(), 4 * (size_t)nl, cudaMemcpyHostToDevice);
-            cudaMemcpy(d_noff, h_noff.data(), 4 * (size_t)(nn + 1), cudaMemcpyHostToDevice);
-            k_scatter<<<blocks(nl, kScatterWarps), 32 * kScatterWarps>>>(d_refs, d_mask, d_off, d_fc, d_noff, nl, d_next);
-            e = cudaGetLastError();
-            if (e == cudaSuccess) e = cudaDeviceSynchronize();
-            if (e != cudaSuccess) {
-                err = std::string("device build: ") + cudaGetErrorString(e);
-                return false;
-            }
-            b_refs.swap(b_next);
-            d_refs = (int *)b_refs.p;
+        if (next_base + 8LL * total.splits >= (int64_t(1) << 31)) {
+            err = "too many nodes for the device build";
+            return false;
         }
-        level.swap(next);
+        auto next = std::make_unique<Level>();
+        next->nodes = 8 * total.splits;
+        next->base = next_base;
+        lv.leaf_base = leaf_total;
+        lv.leaf_refs = total.leaf_refs;
+        float *d_nbox = next->box.get<float>(6 * (size_t)next->nodes);
+        int *d_noff = b_noff.get<int>((size_t)next->nodes + 1);
+        int *d_next = b_next.get<int>((size_t)total.child_refs);
+        int *d_leaf = lv.leaf.get<int>((size_t)total.leaf_refs);
+        if (!d_nbox || !d_noff || !d_next || !d_leaf) { err = "device allocation failed"; return false; }
+        k_emit<<<blocks(nl, 128), 128>>>(d_sums, d_tot, d_off, d_split, d_occ, d_sub, d_lbox, nl, leaf_total, next_base, d_box, d_child,
+                                         d_fc, d_first, d_count, d_noff, d_nbox);
+        if (nr > 0) k_leaf_refs<<<blocks(nr, 256), 256>>>(d_sums, d_tot, d_refs, d_owner, d_off, d_split, nr, d_leaf);
+        if (next->nodes > 0)
+            k_scatter<<<blocks(nl, kScatterWarps), 32 * kScatterWarps>>>(d_refs, d_mask, d_off, d_fc, d_noff, nl, d_next);
+        leaf_total += total.leaf_refs;
+        next_base += next->nodes;
+        nr = (int)total.child_refs;
+        b_refs.swap(b_next);
+        d_refs = (int *)b_refs.p;
+        b_off.swap(b_noff);
+        if (next->nodes == 0) {
+            out.depth = depth;
+            break;
+        }
+        levels.push_back(std::move(next));
     }
 
-    // bottom-up reduce of inner nodes, deeper first (reduceNode(0, false)), as the host builder
-    const int64_t nn = (int64_t)boxes.size();
-    for (int64_t i = nn - 1; i >= 0; i--) {
-        if (child[i] < 0) continue;
-        P3 lo = boxes[i].hi, hi = boxes[i].lo;
-        for (int c = 0; c < 8; c++) {
-            const Bx &cb = boxes[child[i] + c];
-            lo = mk(std::fmin(lo.x, cb.lo.x), std::fmin(lo.y, cb.lo.y), std::fmin(lo.z, cb.lo.z));
-            hi = mk(std::fmax(hi.x, cb.hi.x), std::fmax(hi.y, cb.hi.y), std::fmax(hi.z, cb.hi.z));
-        }
-        boxes[i] = shrink(boxes[i], lo, hi, E);
+    for (int depth = out.depth - 1; depth >= 0; depth--) {
+        Level &lv = *levels[depth], &nx = *levels[depth + 1];
+        k_reduce<<<blocks(lv.nodes, 128), 128>>>((float *)lv.box.p, (const int *)lv.child.p, lv.nodes, nx.base, (const float *)nx.box.p, E);
     }
-    if (root_child >= 0) {
-        P3 lo = root_box.hi, hi = root_box.lo;
-        for (int c = 0; c < 8; c++) {
-            const Bx &cb = boxes[root_child + c];
-            lo = mk(std::fmin(lo.x, cb.lo.x), std::fmin(lo.y, cb.lo.y), std::fmin(lo.z, cb.lo.z));
-            hi = mk(std::fmax(hi.x, cb.hi.x), std::fmax(hi.y, cb.hi.y), std::fmax(hi.z, cb.hi.z));
-        }
-        root_box = shrink(root_box, lo, hi, E);
-    }
+
+    // the finished tree
+    const int64_t nn = next_base;
     out.node_count = nn;
     out.node_lo.resize(3 * nn);
     out.node_hi.resize(3 * nn);
-    out.node_child = std::move(child);
+    out.node_child.resize(nn);
     out.node_leaf_first.resize(nn);
-    out.node_leaf_count = std::move(leaf_cnt);
-    for (int64_t i = 0; i < nn; i++) {
-        out.node_lo[3 * i] = boxes[i].lo.x; out.node_lo[3 * i + 1] = boxes[i].lo.y; out.node_lo[3 * i + 2] = boxes[i].lo.z;
-        out.node_hi[3 * i] = boxes[i].hi.x; out.node_hi[3 * i + 1] = boxes[i].hi.y; out.node_hi[3 * i + 2] = boxes[i].hi.z;
-        out.node_leaf_first[i] = leaf_lo[i];
+    out.node_leaf_count.resize(nn);
+    out.leaf_refs.resize((size_t)leaf_total);
+    DevBuf b_lo, b_hi;
+    float *d_lo = b_lo.get<float>(3 * (size_t)nn), *d_hi = b_hi.get<float>(3 * (size_t)nn);
+    if (!d_lo || !d_hi) { err = "device allocation failed"; return false; }
+    cudaError_t e = cudaGetLastError();
+    auto fetch = [&](void *dst, const void *src, size_t bytes) {
+        if (e == cudaSuccess && bytes) e = cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost);
+    };
+    for (size_t d = 0; d < levels.size(); d++) {
+        const Level &lv = *levels[d];
+        fetch(out.leaf_refs.data() + lv.leaf_base, lv.leaf.p, 4 * (size_t)lv.leaf_refs);
+        if (d == 0) {
+            float b[6];
+            int child, count;
+            fetch(b, lv.box.p, sizeof(b));
+            fetch(&child, lv.child.p, sizeof(child));
+            fetch(&count, lv.count.p, sizeof(count));
+            for (int k = 0; k < 3; k++) { out.root_lo[k] = b[k]; out.root_hi[k] = b[3 + k]; }
+            out.root_child = child;
+            out.root_leaf_first = 0;
+            out.root_leaf_count = count;
+            continue;
+        }
+        k_finish<<<blocks(3LL * lv.nodes, 256), 256>>>((const float *)lv.box.p, lv.nodes, d_lo + 3 * (size_t)lv.base, d_hi + 3 * (size_t)lv.base);
+        fetch(out.node_child.data() + lv.base, lv.child.p, 4 * (size_t)lv.nodes);
+        static_assert(sizeof(long long) == sizeof(int64_t), "leaf_first is copied as it is");
+        fetch(out.node_leaf_first.data() + lv.base, lv.first.p, 8 * (size_t)lv.nodes);
+        fetch(out.node_leaf_count.data() + lv.base, lv.count.p, 4 * (size_t)lv.nodes);
     }
-    out.root_lo[0] = root_box.lo.x; out.root_lo[1] = root_box.lo.y; out.root_lo[2] = root_box.lo.z;
-    out.root_hi[0] = root_box.hi.x; out.root_hi[1] = root_box.hi.y; out.root_hi[2] = root_box.hi.z;
-    out.root_child = root_child;
-    out.root_leaf_first = root_leaf_lo;
-    out.root_leaf_count = root_leaf_cnt;
-    out.depth = max_seen;
+    if (e == cudaSuccess) e = cudaGetLastError();
+    fetch(out.node_lo.data(), d_lo, 12 * (size_t)nn);
+    fetch(out.node_hi.data(), d_hi, 12 * (size_t)nn);
+    if (e != cudaSuccess) {
+        err = std::string("device build: ") + cudaGetErrorString(e);
+        return false;
+    }
     return true;
 }
 
