@@ -16,7 +16,7 @@
 
 #include "../../include/dr_api.h"
 #include "dr_kernels.h"
-#include "octree_build.h"
+#include "octree_device.h"
 #include "dr_internal.h"
 #include "dr_guard.h"
 
@@ -45,19 +45,13 @@ cudaError_t upload(T **dst, const T *src, size_t count) {
     return cudaMemcpy(*dst, src, sizeof(T) * count, cudaMemcpyHostToDevice);
 }
 
-// normalised Triangle::normal() = (c - a) x (b - a) (flat shading default)
-void flat_normal(const float *p, float out[3]) {
-    float ax = p[0], ay = p[1], az = p[2];
-    float cax = p[6] - ax, cay = p[7] - ay, caz = p[8] - az;
-    float bax = p[3] - ax, bay = p[4] - ay, baz = p[5] - az;
-    float x = cay * baz - bay * caz;
-    float y = bax * caz - cax * baz;
-    float z = cax * bay - bax * cay;
-    float im = 1.0f / std::sqrt(x * x + y * y + z * z);
-    out[0] = x * im;
-    out[1] = y * im;
-    out[2] = z * im;
-}
+// Frees device scratch at the end of a scope.
+struct DeviceScratch {
+    std::vector<void *> p;
+    ~DeviceScratch() {
+        for (void *q : p) cudaFree(q);
+    }
+};
 
 }  // namespace
 
@@ -393,7 +387,8 @@ dr_status dr_scene_create(const float *xyz, const float *nrm, const int32_t *mat
         opt.device = bp->device_build != 0;
     }
     std::string berr;
-    if (!(opt.device ? drb::build_octree_gpu(sc->xyz.data(), n, opt, sc->tree, berr)
+    drb::DeviceTree dt;
+    if (!(opt.device ? drb::build_octree_gpu(sc->xyz.data(), n, opt, sc->tree, &dt, berr)
                      : drb::build_octree(sc->xyz.data(), n, opt, sc->tree))) {
         delete sc;
         return fail(opt.device ? DR_E_CUDA : DR_E_ARG, "dr_scene_create: octree build failed" + (berr.empty() ? std::string() : ": " + berr));
@@ -402,30 +397,6 @@ dr_status dr_scene_create(const float *xyz, const float *nrm, const int32_t *mat
     if (T.node_count >= (int64_t(1) << 24)) {
         delete sc;
         return fail(DR_E_CAPACITY, "dr_scene_create: octree exceeds 2^24 nodes");
-    }
-    // pack nodes: {lo, first child | ~first ref}, {hi, ref count}
-    std::vector<float4> nodes(2 * (size_t)T.node_count);
-    for (int64_t i = 0; i < T.node_count; i++) {
-        int w = T.node_child[i] >= 0 ? T.node_child[i] : ~(int)T.node_leaf_first[i];
-        int c = T.node_child[i] >= 0 ? 0 : T.node_leaf_count[i];
-        float wf, cf;
-        std::memcpy(&wf, &w, 4);
-        std::memcpy(&cf, &c, 4);
-        nodes[2 * i] = make_float4(T.node_lo[3 * i], T.node_lo[3 * i + 1], T.node_lo[3 * i + 2], wf);
-        nodes[2 * i + 1] = make_float4(T.node_hi[3 * i], T.node_hi[3 * i + 1], T.node_hi[3 * i + 2], cf);
-    }
-    std::vector<float4> tris(3 * (size_t)n), nrms(3 * (size_t)n);
-    for (int64_t i = 0; i < n; i++) {
-        const float *p = &sc->xyz[9 * i];
-        for (int k = 0; k < 3; k++) tris[3 * i + k] = make_float4(p[3 * k], p[3 * k + 1], p[3 * k + 2], 0.0f);
-        if (nrm) {
-            const float *q = nrm + 9 * i;
-            for (int k = 0; k < 3; k++) nrms[3 * i + k] = make_float4(q[3 * k], q[3 * k + 1], q[3 * k + 2], 0.0f);
-        } else {
-            float fn[3];
-            flat_normal(p, fn);
-            for (int k = 0; k < 3; k++) nrms[3 * i + k] = make_float4(fn[0], fn[1], fn[2], 0.0f);
-        }
     }
     std::vector<drd::Material> dm(std::max(n_mats, 1));
     std::memset(dm.data(), 0, sizeof(drd::Material) * dm.size());
@@ -465,45 +436,68 @@ dr_status dr_scene_create(const float *xyz, const float *nrm, const int32_t *mat
         if (l.type == DR_LIGHT_SPOTLIGHT) spotlight_state(l, d);
     }
 
-    std::vector<float> gbox, gbox_ref;
-    group_planes(T, gbox, gbox_ref);
+    // the tree's arrays, if it was built on the host
+    cudaError_t e = cudaSuccess;
+    if (!dt.xyz) {
+        e = upload(&dt.xyz, sc->xyz.data(), sc->xyz.size());
+        if (e == cudaSuccess) e = upload(&dt.lo, T.node_lo.data(), T.node_lo.size());
+        if (e == cudaSuccess) e = upload(&dt.hi, T.node_hi.data(), T.node_hi.size());
+        if (e == cudaSuccess) e = upload(&dt.child, T.node_child.data(), T.node_child.size());
+        if (e == cudaSuccess) e = upload(&dt.leaf_first, reinterpret_cast<const long long *>(T.node_leaf_first.data()), T.node_leaf_first.size());
+        if (e == cudaSuccess) e = upload(&dt.leaf_count, T.node_leaf_count.data(), T.node_leaf_count.size());
+        if (e == cudaSuccess) e = upload(&dt.refs, T.leaf_refs.data(), T.leaf_refs.size());
+    }
+    // where each level's nodes begin: a level's inner nodes have 8 children each in the next
+    std::vector<int64_t> levels{0};
+    for (int64_t end = T.node_count > 0 ? 8 : 0; end > levels.back();) {
+        int64_t inner = 0;
+        for (int64_t i = levels.back(); i < end; i++) inner += T.node_child[i] >= 0;
+        levels.push_back(end);
+        end += 8 * inner;
+    }
+    float reach = 0.0f;
+    for (int k = 0; k < 3; k++) reach = std::fmax(reach, std::fmax(std::fabs(T.root_lo[k]), std::fabs(T.root_hi[k])));
+
+    DeviceScratch scratch;
+    auto take = [&](auto **p, size_t count, bool keep = true) {   // device memory of the scene, or of this call
+        if (e != cudaSuccess || count == 0) return;
+        e = cudaMalloc((void **)p, sizeof(**p) * count);
+        if (e == cudaSuccess) (keep ? sc->allocs : scratch.p).push_back(*p);
+    };
+    auto give = [&](auto **p, const auto *src, size_t count, bool keep = true) {
+        take(p, count, keep);
+        if (e == cudaSuccess && count) e = cudaMemcpy(*p, src, sizeof(**p) * count, cudaMemcpyHostToDevice);
+    };
+    const size_t nn = (size_t)T.node_count, n_refs = T.leaf_refs.size();
     float4 *d_nodes = nullptr, *d_gbox = nullptr, *d_gbox_ref = nullptr, *d_groups = nullptr, *d_leaf = nullptr, *d_tris = nullptr, *d_nrms = nullptr;
+    float4 *d_fit = nullptr;
+    float *d_nrm = nullptr;
     int *d_mat = nullptr;
     drd::Material *d_mats = nullptr;
     drd::Light *d_lights = nullptr;
-    cudaError_t e = upload(&d_nodes, nodes.data(), nodes.size());
-    if (e == cudaSuccess) { sc->allocs.push_back(d_nodes); e = upload(&d_gbox, (const float4 *)gbox.data(), gbox.size() / 4); }
-    if (e == cudaSuccess) { sc->allocs.push_back(d_gbox); e = upload(&d_gbox_ref, (const float4 *)gbox_ref.data(), gbox_ref.size() / 4); }
-    if (e == cudaSuccess) { sc->allocs.push_back(d_gbox_ref); e = upload(&d_tris, tris.data(), tris.size()); }
-    if (e == cudaSuccess) { sc->allocs.push_back(d_tris); e = upload(&d_nrms, nrms.data(), nrms.size()); }
-    if (e == cudaSuccess) { sc->allocs.push_back(d_nrms); e = upload(&d_mat, sc->mat_id.data(), sc->mat_id.size()); }
-    if (e == cudaSuccess) { sc->allocs.push_back(d_mat); e = upload(&d_mats, dm.data(), dm.size()); }
-    if (e == cudaSuccess) { sc->allocs.push_back(d_mats); e = upload(&d_lights, dl.data(), dl.size()); }
-    if (e == cudaSuccess) sc->allocs.push_back(d_lights);
-    const size_t n_refs = T.leaf_refs.size();
-    int *d_refs = nullptr;
-    if (e == cudaSuccess) e = upload(&d_refs, T.leaf_refs.data(), n_refs);
-    if (e == cudaSuccess && n_refs) e = cudaMalloc((void **)&d_leaf, sizeof(float4) * drd::kLeafTriF4 * n_refs);
-    if (e == cudaSuccess && n_refs) {
-        sc->allocs.push_back(d_leaf);
-        e = drk::launch_leaf_tris(d_leaf, d_refs, d_tris, (long long)n_refs, nullptr);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
-    }
-    cudaFree(d_refs);
-    float reach = 0.0f;
-    for (int k = 0; k < 3; k++) reach = std::fmax(reach, std::fmax(std::fabs(T.root_lo[k]), std::fabs(T.root_hi[k])));
-    const int64_t n_groups = T.node_count / 8;
-    if (e == cudaSuccess && n_groups) e = cudaMalloc((void **)&d_groups, sizeof(float4) * drd::kRecordF4 * (size_t)n_groups);
-    if (e == cudaSuccess && n_groups) {
-        sc->allocs.push_back(d_groups);
-        e = drk::launch_group_records(d_groups, d_nodes, d_gbox, n_groups, reach * drd::kRecordPad, nullptr);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
-    }
+    take(&d_nodes, 2 * nn);
+    take(&d_gbox, 12 * (nn / 8));
+    take(&d_gbox_ref, 12 * (nn / 8));
+    take(&d_groups, drd::kRecordF4 * (nn / 8));
+    take(&d_leaf, drd::kLeafTriF4 * n_refs);
+    take(&d_tris, 3 * (size_t)n);
+    take(&d_nrms, 3 * (size_t)n);
+    take(&d_fit, 2 * nn, false);
+    give(&d_mat, sc->mat_id.data(), sc->mat_id.size());
+    give(&d_mats, dm.data(), dm.size());
+    give(&d_lights, dl.data(), dl.size());
+    if (nrm) give(&d_nrm, nrm, 9 * (size_t)n, false);
+    if (e == cudaSuccess) e = drk::launch_scene_tris(d_tris, d_nrms, dt.xyz, d_nrm, n, nullptr);
+    if (e == cudaSuccess) e = drk::launch_leaf_tris(d_leaf, dt.refs, d_tris, (long long)n_refs, nullptr);
+    if (e == cudaSuccess)
+        e = drk::launch_scene_nodes(d_nodes, d_gbox, d_gbox_ref, d_groups, d_fit, dt.lo, dt.hi, dt.child, dt.leaf_first, dt.leaf_count, levels,
+                                    reach * drd::kRecordPad, nullptr);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) {
         delete sc;
         return cuda_fail(e, "dr_scene_create: upload");
     }
-    sc->node_f4 = (int64_t)nodes.size();
+    sc->node_f4 = 2 * T.node_count;
     sc->leaf_f4 = (int64_t)(drd::kLeafTriF4 * n_refs);
     drd::Scene &S = sc->dev;
     S.nodes = d_nodes;
@@ -673,7 +667,7 @@ dr_status dr_octree_create_host(const float *xyz, int32_t n, const dr_build_para
         opt.device = bp->device_build != 0;
     }
     std::string berr;
-    if (!(opt.device ? drb::build_octree_gpu(xyz, n, opt, t->tree, berr) : drb::build_octree(xyz, n, opt, t->tree))) {
+    if (!(opt.device ? drb::build_octree_gpu(xyz, n, opt, t->tree, nullptr, berr) : drb::build_octree(xyz, n, opt, t->tree))) {
         delete t;
         return fail(opt.device ? DR_E_CUDA : DR_E_ARG, "dr_octree_create_host: build failed" + (berr.empty() ? std::string() : ": " + berr));
     }

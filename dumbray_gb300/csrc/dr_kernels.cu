@@ -1141,6 +1141,77 @@ __global__ void k_resolve(WaveArgs A, int total_slots) {
     }
 }
 
+// ---- scene records from a built tree ----------------------------------------------------------
+// Triangles and corner normals by id, one thread per corner; without normals the flat one.
+__global__ void k_scene_tris(float4 *tris, float4 *nrms, const float *xyz, const float *nrm, int n) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= 3LL * n) return;
+    const float *p = xyz + 3 * i;
+    tris[i] = make_float4(p[0], p[1], p[2], 0.0f);
+    if (nrm) {
+        const float *q = nrm + 3 * i;
+        nrms[i] = make_float4(q[0], q[1], q[2], 0.0f);
+        return;
+    }
+    const float *t = xyz + 9 * (i / 3);
+    const f3 a = mkf3(t[0], t[1], t[2]), b = mkf3(t[3], t[4], t[5]), c = mkf3(t[6], t[7], t[8]);
+    const f3 m = xcross(xsub(c, a), xsub(b, a));   // Triangle::normal()
+    const float im = __fdiv_rn(1.0f, xmag(m));
+    nrms[i] = make_float4(__fmul_rn(m.x, im), __fmul_rn(m.y, im), __fmul_rn(m.z, im), 0.0f);
+}
+
+// Nodes: {lo, first child | ~first reference}, {hi, reference count}.
+__global__ void k_scene_nodes(float4 *nodes, const float *lo, const float *hi, const int *child, const long long *first, const int *count,
+                              long long n) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int c = child[i];
+    nodes[2 * i] = make_float4(lo[3 * i], lo[3 * i + 1], lo[3 * i + 2], __int_as_float(c >= 0 ? c : ~(int)first[i]));
+    nodes[2 * i + 1] = make_float4(hi[3 * i], hi[3 * i + 1], hi[3 * i + 2], __int_as_float(c >= 0 ? 0 : count[i]));
+}
+
+// Boxes refitted to the non-empty leaves below, for one level of nodes whose children are done: a leaf's
+// own box, an inner node's union of its children's; w of {lo, w} = whether there is any.
+constexpr float kFarPlane = 1e30f;
+__global__ void k_scene_refit(float4 *fit, const float *lo, const float *hi, const int *child, const int *count, long long begin, long long end) {
+    const long long i = begin + blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= end) return;
+    f3 l, h;
+    bool live = false;
+    if (child[i] < 0) {
+        live = count[i] > 0;
+        l = mkf3(lo[3 * i], lo[3 * i + 1], lo[3 * i + 2]);
+        h = mkf3(hi[3 * i], hi[3 * i + 1], hi[3 * i + 2]);
+    } else {
+        l = mkf3(kFarPlane, kFarPlane, kFarPlane);
+        h = mkf3(-kFarPlane, -kFarPlane, -kFarPlane);
+        for (int c = 0; c < 8; c++) {
+            const long long j = (long long)child[i] + c;
+            const float4 a = fit[2 * j], b = fit[2 * j + 1];
+            if (a.w == 0.0f) continue;
+            live = true;
+            l = mkf3(fminf(l.x, a.x), fminf(l.y, a.y), fminf(l.z, a.z));
+            h = mkf3(fmaxf(h.x, b.x), fmaxf(h.y, b.y), fmaxf(h.z, b.z));
+        }
+    }
+    fit[2 * i] = make_float4(l.x, l.y, l.z, live ? 1.0f : 0.0f);
+    fit[2 * i + 1] = make_float4(h.x, h.y, h.z, 0.0f);
+}
+
+// Child planes of every group (Scene::gbox, gbox_ref): one thread per group and plane.
+__global__ void k_scene_planes(float *gbox, float *gbox_ref, const float4 *fit, const float *lo, const float *hi, const int *child, const int *count,
+                               long long n_groups) {
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (t >= 48 * n_groups) return;
+    const long long g = t / 48;
+    const int j = (int)(t - 48 * g), c = j & 7, axis = (j >> 3) % 3;
+    const long long i = 8 * g + c;
+    const float *box = j < 24 ? lo : hi;
+    const float4 l = fit[2 * i], h = fit[2 * i + 1], f = j < 24 ? l : h;
+    gbox_ref[t] = child[i] < 0 && count[i] == 0 ? kFarPlane : box[3 * i + axis];
+    gbox[t] = l.w == 0.0f ? kFarPlane : axis == 0 ? f.x : axis == 1 ? f.y : f.z;
+}
+
 // Leaf references (kLeafTriF4 layout) from the triangles: one thread per reference.
 __global__ void k_leaf_tris(float4 *dst, const int *refs, const float4 *tris, long long n_refs) {
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < n_refs; r += (long long)gridDim.x * blockDim.x) {
@@ -1453,6 +1524,26 @@ cudaError_t launch_rebase_nodes(float4 *dst, const float4 *src, long long n_node
     const int grid = (int)std::min<long long>((n_nodes + 255) / 256, (long long)sm_count() * 8);
     drd::k_rebase_nodes<<<grid, 256, 0, stream>>>(dst, src, n_nodes, group_off, leaf_off);
     return cudaGetLastError();
+}
+
+cudaError_t launch_scene_tris(float4 *tris, float4 *nrms, const float *xyz, const float *nrm, int n, cudaStream_t stream) {
+    if (n <= 0) return cudaSuccess;
+    drd::k_scene_tris<<<(unsigned)((3LL * n + 255) / 256), 256, 0, stream>>>(tris, nrms, xyz, nrm, n);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_scene_nodes(float4 *nodes, float4 *gbox, float4 *gbox_ref, float4 *groups, float4 *fit, const float *lo, const float *hi,
+                               const int *child, const long long *first, const int *count, const std::vector<int64_t> &levels, float pad,
+                               cudaStream_t stream) {
+    const int64_t n = levels.back(), n_groups = n / 8;
+    if (n <= 0) return cudaSuccess;
+    drd::k_scene_nodes<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(nodes, lo, hi, child, first, count, n);
+    for (size_t d = levels.size() - 1; d-- > 0;)
+        drd::k_scene_refit<<<(unsigned)((levels[d + 1] - levels[d] + 127) / 128), 128, 0, stream>>>(fit, lo, hi, child, count, levels[d], levels[d + 1]);
+    drd::k_scene_planes<<<(unsigned)((48 * n_groups + 255) / 256), 256, 0, stream>>>(reinterpret_cast<float *>(gbox), reinterpret_cast<float *>(gbox_ref),
+                                                                                    fit, lo, hi, child, count, n_groups);
+    const cudaError_t e = cudaGetLastError();
+    return e != cudaSuccess ? e : launch_group_records(groups, nodes, gbox, n_groups, pad, stream);
 }
 
 cudaError_t launch_leaf_tris(float4 *dst, const int *refs, const float4 *tris, long long n_refs, cudaStream_t stream) {

@@ -107,6 +107,13 @@ cudaError_t launch_wave(const WaveDesc &W, cudaStream_t stream, long long *launc
 // index 8 * group_off), adding the offsets to child node and first-leaf-reference indices.
 cudaError_t launch_rebase_nodes(float4 *dst, const float4 *src, long long n_nodes, int group_off, int leaf_off,
                                 cudaStream_t stream);
+// Scene records from a built tree in device memory.  Triangles and corner normals (flat without `nrm`);
+// nodes, child planes and group records: `levels` = where each level's nodes begin, breadth first, and
+// the node count at the end; `fit` is scratch of 2 float4 per node; boxes of the records widened by `pad`.
+cudaError_t launch_scene_tris(float4 *tris, float4 *nrms, const float *xyz, const float *nrm, int n, cudaStream_t stream);
+cudaError_t launch_scene_nodes(float4 *nodes, float4 *gbox, float4 *gbox_ref, float4 *groups, float4 *fit, const float *lo, const float *hi,
+                               const int *child, const long long *first, const int *count, const std::vector<int64_t> &levels, float pad,
+                               cudaStream_t stream);
 // Leaf references (drd::kLeafTriF4 float4 each) from the triangle ids in leaf order.
 cudaError_t launch_leaf_tris(float4 *dst, const int *refs, const float4 *tris, long long n_refs, cudaStream_t stream);
 // Group records (drd::kRecordF4 float4 each) of a scene from its nodes and refitted planes, boxes

@@ -26,7 +26,7 @@
 #include <string>
 #include <vector>
 
-#include "octree_build.h"
+#include "octree_device.h"
 #include "octree_geom.h"
 
 namespace drb {
@@ -430,6 +430,12 @@ struct DevBuf {
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
     ~DevBuf() { cudaFree(p); }
+    void *release() {
+        void *q = p;
+        p = nullptr;
+        bytes = 0;
+        return q;
+    }
     void swap(DevBuf &o) {
         std::swap(p, o.p);
         std::swap(bytes, o.bytes);
@@ -452,7 +458,7 @@ struct DevBuf {
 
 }  // namespace
 
-bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, FlatOctree &out, std::string &err) {
+bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, FlatOctree &out, DeviceTree *keep, std::string &err) {
     out = FlatOctree();
     if (n <= 0) return true;
     if (n >= (int64_t(1) << 31)) {
@@ -599,40 +605,53 @@ bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, Flat
     out.node_leaf_first.resize(nn);
     out.node_leaf_count.resize(nn);
     out.leaf_refs.resize((size_t)leaf_total);
-    DevBuf b_lo, b_hi;
+    DevBuf b_lo, b_hi, b_child, b_first, b_count, b_leaf;
     float *d_lo = b_lo.get<float>(3 * (size_t)nn), *d_hi = b_hi.get<float>(3 * (size_t)nn);
-    if (!d_lo || !d_hi) { err = "device allocation failed"; return false; }
+    int *d_child = b_child.get<int>((size_t)nn), *d_count = b_count.get<int>((size_t)nn);
+    long long *d_first = b_first.get<long long>((size_t)nn);
+    int *d_leaf = b_leaf.get<int>((size_t)leaf_total);
+    if (!d_lo || !d_hi || !d_child || !d_count || !d_first || !d_leaf) { err = "device allocation failed"; return false; }
     cudaError_t e = cudaGetLastError();
-    auto fetch = [&](void *dst, const void *src, size_t bytes) {
-        if (e == cudaSuccess && bytes) e = cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost);
+    auto copy = [&](void *dst, const void *src, size_t bytes, cudaMemcpyKind kind) {
+        if (e == cudaSuccess && bytes) e = cudaMemcpy(dst, src, bytes, kind);
     };
     for (size_t d = 0; d < levels.size(); d++) {
         const Level &lv = *levels[d];
-        fetch(out.leaf_refs.data() + lv.leaf_base, lv.leaf.p, 4 * (size_t)lv.leaf_refs);
+        copy(d_leaf + lv.leaf_base, lv.leaf.p, 4 * (size_t)lv.leaf_refs, cudaMemcpyDeviceToDevice);
         if (d == 0) {
             float b[6];
-            int child, count;
-            fetch(b, lv.box.p, sizeof(b));
-            fetch(&child, lv.child.p, sizeof(child));
-            fetch(&count, lv.count.p, sizeof(count));
+            copy(b, lv.box.p, sizeof(b), cudaMemcpyDeviceToHost);
+            copy(&out.root_child, lv.child.p, 4, cudaMemcpyDeviceToHost);
+            copy(&out.root_leaf_count, lv.count.p, 4, cudaMemcpyDeviceToHost);
             for (int k = 0; k < 3; k++) { out.root_lo[k] = b[k]; out.root_hi[k] = b[3 + k]; }
-            out.root_child = child;
             out.root_leaf_first = 0;
-            out.root_leaf_count = count;
             continue;
         }
         k_finish<<<blocks(3LL * lv.nodes, 256), 256>>>((const float *)lv.box.p, lv.nodes, d_lo + 3 * (size_t)lv.base, d_hi + 3 * (size_t)lv.base);
-        fetch(out.node_child.data() + lv.base, lv.child.p, 4 * (size_t)lv.nodes);
-        static_assert(sizeof(long long) == sizeof(int64_t), "leaf_first is copied as it is");
-        fetch(out.node_leaf_first.data() + lv.base, lv.first.p, 8 * (size_t)lv.nodes);
-        fetch(out.node_leaf_count.data() + lv.base, lv.count.p, 4 * (size_t)lv.nodes);
+        copy(d_child + lv.base, lv.child.p, 4 * (size_t)lv.nodes, cudaMemcpyDeviceToDevice);
+        copy(d_first + lv.base, lv.first.p, 8 * (size_t)lv.nodes, cudaMemcpyDeviceToDevice);
+        copy(d_count + lv.base, lv.count.p, 4 * (size_t)lv.nodes, cudaMemcpyDeviceToDevice);
     }
     if (e == cudaSuccess) e = cudaGetLastError();
-    fetch(out.node_lo.data(), d_lo, 12 * (size_t)nn);
-    fetch(out.node_hi.data(), d_hi, 12 * (size_t)nn);
+    static_assert(sizeof(long long) == sizeof(int64_t), "leaf_first is copied as it is");
+    copy(out.node_lo.data(), d_lo, 12 * (size_t)nn, cudaMemcpyDeviceToHost);
+    copy(out.node_hi.data(), d_hi, 12 * (size_t)nn, cudaMemcpyDeviceToHost);
+    copy(out.node_child.data(), d_child, 4 * (size_t)nn, cudaMemcpyDeviceToHost);
+    copy(out.node_leaf_first.data(), d_first, 8 * (size_t)nn, cudaMemcpyDeviceToHost);
+    copy(out.node_leaf_count.data(), d_count, 4 * (size_t)nn, cudaMemcpyDeviceToHost);
+    copy(out.leaf_refs.data(), d_leaf, 4 * (size_t)leaf_total, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) {
         err = std::string("device build: ") + cudaGetErrorString(e);
         return false;
+    }
+    if (keep) {
+        keep->xyz = (float *)b_xyz.release();
+        keep->lo = (float *)b_lo.release();
+        keep->hi = (float *)b_hi.release();
+        keep->child = (int32_t *)b_child.release();
+        keep->leaf_first = (long long *)b_first.release();
+        keep->leaf_count = (int32_t *)b_count.release();
+        keep->refs = (int32_t *)b_leaf.release();
     }
     return true;
 }
