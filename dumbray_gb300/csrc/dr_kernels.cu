@@ -85,13 +85,6 @@ __device__ __forceinline__ int block_alloc_by_octant(int *counter, bool want, f3
     return want ? sh.out + sh.cnt[wid][oct] + __popc(mine & ((1u << lane_id()) - 1u)) : -1;
 }
 
-// Warp-level work fetch from a dynamic counter; returns the base index (warp-uniform).
-__device__ __forceinline__ int warp_fetch(int *counter) {
-    int base = 0;
-    if (lane_id() == 0) base = atomicAdd(counter, 32);
-    return __shfl_sync(0xFFFFFFFFu, base, 0);
-}
-
 // Chunked work fetch from a device counter (warp-uniform).  The chunk shrinks with the queue: about 4
 // chunks per resident warp, between 32 and kChunk rays, and the rays of one warp when there are not
 // enough for all lanes (warp_width), so short queues (late bounces, shadow queues) still spread over
@@ -209,7 +202,6 @@ struct Ctrl {
     int kept_count[kMaxBounceSlots];      // those of them that continue when the carry region is full
     int carry_count;                      // continuing reference photons moved to the carry region
     int fetch_carry;
-    int fetch_camera;
     int error;
 };
 
@@ -337,13 +329,16 @@ __device__ __forceinline__ int job_of_path(const WaveArgs &A, long long g) {
     return lo;
 }
 
+// One thread per path, blocks in grid strides; valid paths are compacted with one atomic a block.  (A
+// fetch and an allocation a warp were 262k atomics on two addresses for a 4Mi-path wave, and the path
+// index a 64-bit division: 0.25 ms against 0.04 ms of queue writes.)
+constexpr int kCameraThreads = 256;
 template <bool MULTI>
-__global__ void __launch_bounds__(256) k_camera(WaveArgs A) {
-    Ctrl *C = A.ctrl;
-    for (;;) {
-        int base = warp_fetch(&C->fetch_camera);
-        if (base >= A.wave_count) break;
-        int i = base + (int)lane_id();
+__global__ void __launch_bounds__(kCameraThreads) k_camera(WaveArgs A) {
+    __shared__ int counts[kCameraThreads / 32], block_at;
+    const int warp = (int)(threadIdx.x >> 5);
+    for (int base = (int)blockIdx.x * kCameraThreads; base < A.wave_count; base += (int)gridDim.x * kCameraThreads) {
+        const int i = base + (int)threadIdx.x;
         bool valid = i < A.wave_count;
         f3 o = f3{0, 0, 0}, d = f3{0, 0, 1};
         c3 filt = mkc(0, 0, 0);
@@ -353,8 +348,8 @@ __global__ void __launch_bounds__(256) k_camera(WaveArgs A) {
             long long g = A.wave_begin + i;
             job = job_of_path<MULTI>(A, g);
             const Item &I = job_of<MULTI>(A, job);
-            long long lp = g - I.path_begin;
-            int s = (int)(lp / I.n_slots);
+            const long long lp = g - I.path_begin;
+            const int s = lp >> 32 ? (int)(lp / I.n_slots) : (int)((uint32_t)lp / (uint32_t)I.n_slots);
             int lslot = (int)(lp - (long long)s * I.n_slots);
             slot = I.slot_begin + lslot;
             int blk = I.start_block + lslot / (DR_BLOCK_W * DR_BLOCK_H);
@@ -370,14 +365,25 @@ __global__ void __launch_bounds__(256) k_camera(WaveArgs A) {
                 valid = lens_ray(I, x, y, s, key, o, d, filt);
             }
         }
-        int w = warp_alloc(&C->ray_count[0], valid);
+        const unsigned mine = __ballot_sync(0xFFFFFFFFu, valid);
+        if (lane_id() == 0) counts[warp] = __popc(mine);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int total = 0;
+            for (int v = 0; v < kCameraThreads / 32; v++) total += counts[v];
+            block_at = total ? atomicAdd(&A.ctrl->ray_count[0], total) : 0;
+        }
+        __syncthreads();
         if (valid) {
+            int w = block_at + __popc(mine & ((1u << lane_id()) - 1u));
+            for (int v = 0; v < warp; v++) w += counts[v];
             Queue &Q = A.q[0];
             Q.p0[w] = make_float4(o.x, o.y, o.z, __int_as_float(slot));
             Q.p1[w] = make_float4(d.x, d.y, d.z, __uint_as_float(sample));
             Q.p2[w] = make_float4(filt.r, filt.g, filt.b, 0.0f);
             Q.p3[w] = make_int4(-1, 1 | (i << 1), pixel, job);
         }
+        __syncthreads();   // counts and block_at are read
     }
 }
 
@@ -1450,7 +1456,7 @@ template <bool MULTI, int TT, int TB>
 static void launch_wave_t(const WaveDesc &W, const WaveArgs &A, cudaStream_t stream, Profiler &P, bool count, long long &nl) {
     const int grid = sm_count() * 8;
     P.begin(KC_CAMERA, stream);
-    k_camera<MULTI><<<grid, 256, 0, stream>>>(A);
+    k_camera<MULTI><<<std::min(grid, (W.wave_count + kCameraThreads - 1) / kCameraThreads), kCameraThreads, 0, stream>>>(A);
     P.end(KC_CAMERA, stream);
     nl++;
     const int tgrid = sm_count() * TB;   // one persistent block per slot
