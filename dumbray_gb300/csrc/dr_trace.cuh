@@ -37,7 +37,7 @@ enum : int { kIdle = 0, kTrav = 1, kLeaf = 2, kDone = 3 };
 // A warp's shared slots, one per lane.
 struct WarpSlots {
     float4 o[32];                    // origin, ignored triangle
-    float4 d[32];                    // direction
+    float4 d[32];                    // direction, rounding margin of hit points (point_margin)
     unsigned long long key[32];      // nearest hit of the current leaf: distance bits << 32 | list position
     int2 task[32];                   // round's k-th owner: its lane, its first reference - its first task
 };
@@ -68,15 +68,14 @@ struct StackOf<true> {
 };
 
 // Starts a ray: root leaf, root miss, or the root's children tested (Octree.impl.cuh:175-190).
-template <bool COUNT>
+template <bool COUNT, bool MULTI>
 __device__ __forceinline__ int lane_start(const Scene &S, LaneRay &L, f3 o, f3 d) {
-    const f3 inv = mkf3(__fdiv_rn(1.0f, d.x), __fdiv_rn(1.0f, d.y), __fdiv_rn(1.0f, d.z));
     L.order = (d.z < 0 ? 1 : 0) + (d.y < 0 ? 2 : 0) + (d.x < 0 ? 4 : 0);
     L.sp = 0;
     L.cur = 0;
     if (COUNT) {
         L.o = o;
-        L.inv = inv;
+        L.inv = mkf3(__fdiv_rn(1.0f, d.x), __fdiv_rn(1.0f, d.y), __fdiv_rn(1.0f, d.z));
         L.nb = 0;
         L.nt = 0;
         L.kleaf = 0;
@@ -92,37 +91,47 @@ __device__ __forceinline__ int lane_start(const Scene &S, LaneRay &L, f3 o, f3 d
         }
         return kLeaf;
     }
-    if (COUNT) L.nb++;
-    const bool front = !COUNT || S.front_only != 0;
-    if (slab_hit(S.root_lo[0], S.root_lo[1], S.root_lo[2], S.root_hi[0], S.root_hi[1], S.root_hi[2], o, inv, front)) {
-        if (COUNT) {
+    if constexpr (COUNT) {
+        L.nb++;
+        const bool front = S.front_only != 0;
+        if (slab_hit(S.root_lo[0], S.root_lo[1], S.root_lo[2], S.root_hi[0], S.root_hi[1], S.root_hi[2], o, L.inv, front)) {
             L.cur = ((uint32_t)S.root_child << kCountShift) |
-                    test_group(front ? S.gbox : S.gbox_ref, S.root_child, L.order, o, inv, front);
+                    test_group(front ? S.gbox : S.gbox_ref, S.root_child, L.order, o, L.inv, front);
             L.nb += 8;
-        } else {
-            // a frame whose one child left is the root's group: the first step tests it
-            L.k = ray_slopes(o, d, S.reach);
-            L.cur = never_hits(o, d) ? 0u : 1u;
-            L.links = ((uint32_t)S.root_child << 8) | (1u << L.order);
         }
+    } else {
+        // a frame whose one child left is the root's group: the first step tests it.  The root's own box is
+        // tested when a hit is accepted (leaf_accepts); rays of a batch test it here, where their scene is
+        // at hand.
+        bool enter = !never_hits(o, d);
+        if (MULTI) enter = enter && exact_slab(mkf3(S.root_lo[0], S.root_lo[1], S.root_lo[2]), mkf3(S.root_hi[0], S.root_hi[1], S.root_hi[2]), o, d);
+        L.k = ray_slopes(o, d, S.reach);
+        L.cur = enter ? 1u : 0u;
+        L.links = ((uint32_t)S.root_child << 8) | (1u << L.order);
     }
     return kTrav;
 }
 
-// Whether the nearest hit of a leaf ends the ray (castInLeaf's acceptance): its point lies in the
-// leaf's box (or `anywhere`: an occluder), and the ray passes the exact slab test of that box, which
-// the conservative group tests on the way down stand in for.
-__device__ __forceinline__ bool leaf_accepts(const Scene &S, int node, f3 root_lo, f3 root_hi, f3 o, f3 d, f3 p, bool anywhere) {
+// Whether the nearest hit of a leaf ends the ray (castInLeaf's acceptance): its point lies in the leaf's
+// box (or `anywhere`: an occluder), and the ray passes the exact slab tests of that box and of the root,
+// which the conservative group tests on the way down stand in for.  A point `margin` (point_margin) inside
+// a box settles its slab test: the rounded plane distances then lie on either side of the hit's.  Hardly
+// any hit is nearer to a face than that, so the divisions of the exact test stay out of the way.
+__device__ __forceinline__ bool inside_by(f3 p, f3 l, f3 h, float m) {
+    return p.x >= l.x + m && p.y >= l.y + m && p.z >= l.z + m && p.x <= h.x - m && p.y <= h.y - m && p.z <= h.z - m;
+}
+template <bool ROOT>
+__device__ __forceinline__ bool leaf_accepts(const Scene &S, int node, f3 root_lo, f3 root_hi, f3 o, f3 d, f3 p, float margin, bool anywhere) {
     f3 l = root_lo, h = root_hi;
     if (node >= 0) {
         float4 lo, hi;
         ldg2(S.nodes + 2 * (size_t)node, lo, hi);
         l = f3of(lo);
         h = f3of(hi);
-        const f3 inv = mkf3(__fdiv_rn(1.0f, d.x), __fdiv_rn(1.0f, d.y), __fdiv_rn(1.0f, d.z));
-        if (!slab_hit(l.x, l.y, l.z, h.x, h.y, h.z, o, inv, true)) return false;
     }
-    return anywhere || (p.x >= l.x && p.y >= l.y && p.z >= l.z && p.x <= h.x && p.y <= h.y && p.z <= h.z);
+    if (!anywhere && !inside_by(p, l, h, 0.0f)) return false;
+    if (node < 0) return true;
+    return (inside_by(p, l, h, margin) || exact_slab(l, h, o, d)) && (!ROOT || inside_by(p, root_lo, root_hi, margin) || exact_slab(root_lo, root_hi, o, d));
 }
 
 // Loads entry i of the source into the lane and starts its ray; kIdle when the source has nothing
@@ -134,9 +143,10 @@ __device__ __forceinline__ int restart(const Scene &S, Source &src, int i, LaneR
     f3 o, d;
     if (!src.load(i, o, d, ign, job)) return kIdle;
     ws.o[lane] = make_float4(o.x, o.y, o.z, __int_as_float(ign));
-    ws.d[lane] = make_float4(d.x, d.y, d.z, 0.0f);
+    const Scene &own = MULTI ? src.scene(job) : S;
+    ws.d[lane] = make_float4(d.x, d.y, d.z, point_margin(o, own.reach));
     ws.key[lane] = kNoHit;
-    return lane_start<COUNT>(MULTI ? src.scene(job) : S, L, o, d);
+    return lane_start<COUNT, MULTI>(own, L, o, d);
 }
 
 // Lanes per warp that take rays when `n` rays meet `warps` resident warps.  Fewer rays than lanes
@@ -326,7 +336,8 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ty
             if (key != kNoHit) {
                 const float t = __uint_as_float((unsigned)(key >> 32));
                 const bool occluded = Source::kOccludeBelow > 0.0f && t < Source::kOccludeBelow;
-                const f3 o = f3of(ws.o[lane]), d = f3of(ws.d[lane]), p = xadd(o, xmul(d, t));
+                const float4 dm = ws.d[lane];
+                const f3 o = f3of(ws.o[lane]), d = f3of(dm), p = xadd(o, xmul(d, t));
                 if constexpr (COUNT) {
                     if (occluded || (p.x >= L.lx && p.y >= L.ly && p.z >= L.lz && p.x <= L.hx && p.y <= L.hy && p.z <= L.hz)) {
                         L.nb -= 7 - L.kleaf;
@@ -335,8 +346,8 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ty
                     }
                 } else {
                     const Scene &own = MULTI && L.node < 0 ? src.scene(src.job(cur_i)) : S;
-                    if (leaf_accepts(S, L.node, mkf3(own.root_lo[0], own.root_lo[1], own.root_lo[2]),
-                                     mkf3(own.root_hi[0], own.root_hi[1], own.root_hi[2]), o, d, p, occluded))
+                    if (leaf_accepts<!MULTI>(S, L.node, mkf3(own.root_lo[0], own.root_lo[1], own.root_lo[2]),
+                                             mkf3(own.root_hi[0], own.root_hi[1], own.root_hi[2]), o, d, p, dm.w, occluded))
                         mode = kDone;
                 }
                 if (mode != kDone) ws.key[lane] = kNoHit;
