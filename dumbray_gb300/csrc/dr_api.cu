@@ -506,6 +506,7 @@ dr_status dr_scene_create(const float *xyz, const float *nrm, const int32_t *mat
     S.groups = d_groups;
     S.reach = reach;
     S.leaf_tris = d_leaf;
+    S.leaf_half = (int64_t)n_refs;
     S.tris = d_tris;
     S.nrms = d_nrms;
     S.mat_id = d_mat;
@@ -1201,9 +1202,9 @@ static dr_status build_arena(dr_batch *b) {
         e = cudaMalloc((void **)&b->arena_groups, sizeof(float4) * drd::kRecordF4 * (size_t)std::max<int64_t>(nodes / 16, 1));
     for (size_t k = 0; k < uniq.size() && e == cudaSuccess; k++) {
         const dr_scene *sc = uniq[k];
-        if (sc->leaf_f4)
-            e = cudaMemcpy(b->arena_leaf + drd::kLeafTriF4 * leaf_off[k], sc->dev.leaf_tris, sizeof(float4) * (size_t)sc->leaf_f4,
-                           cudaMemcpyDeviceToDevice);
+        for (int64_t h = 0; h < 2 && sc->leaf_f4 && e == cudaSuccess; h++)   // first halves, second halves
+            e = cudaMemcpy(b->arena_leaf + 2 * (h * (leaf / drd::kLeafTriF4) + leaf_off[k]), sc->dev.leaf_tris + 2 * h * sc->dev.leaf_half,
+                           sizeof(float4) * (size_t)(sc->leaf_f4 / 2), cudaMemcpyDeviceToDevice);
         if (e == cudaSuccess && sc->node_f4)
             e = cudaMemcpy(b->arena_gbox + 12 * (node_off[k] / 8), sc->dev.gbox, sizeof(float4) * 12 * (size_t)(sc->node_f4 / 16),
                            cudaMemcpyDeviceToDevice);
@@ -1229,6 +1230,7 @@ static dr_status build_arena(dr_batch *b) {
         S.groups = b->arena_groups;
         S.gbox_ref = b->arena_gbox;   // batches do not run the counting traversal
         S.leaf_tris = b->arena_leaf;
+        S.leaf_half = leaf / drd::kLeafTriF4;
         if (S.root_child >= 0) S.root_child += (int)(node_off[k] / 8);
         S.root_leaf_first += (int)leaf_off[k];
     }

@@ -1284,11 +1284,11 @@ __global__ void k_leaf_tris(float4 *dst, const int *refs, const float4 *tris, lo
         const TriV t = load_tri(tris, id);
         const f3 ab = xsub(t.b, t.a), bc = xsub(t.c, t.b), ca = xsub(t.a, t.c);
         const f3 n = xcross(ab, xsub(t.c, t.a));
-        float4 *q = dst + r * kLeafTriF4;
-        q[0] = make_float4(t.a.x, t.b.x, t.a.y, t.b.y);
-        q[1] = make_float4(t.a.z, t.b.z, t.c.x, t.c.y);
-        q[2] = make_float4(t.c.z, n.x, n.y, n.z);
-        q[3] = make_float4(edge_limit(ab, ca), edge_limit(bc, ab), edge_limit(ca, bc), __int_as_float(id));
+        float4 *p = dst + 2 * r, *q = dst + 2 * (n_refs + r);
+        p[0] = make_float4(t.a.x, t.b.x, t.a.y, t.b.y);
+        p[1] = make_float4(t.a.z, t.b.z, t.c.x, t.c.y);
+        q[0] = make_float4(t.c.z, n.x, n.y, n.z);
+        q[1] = make_float4(edge_limit(ab, ca), edge_limit(bc, ab), edge_limit(ca, bc), __int_as_float(id));
     }
 }
 

@@ -114,7 +114,8 @@ cudaError_t launch_scene_tris(float4 *tris, float4 *nrms, const float *xyz, cons
 cudaError_t launch_scene_nodes(float4 *nodes, float4 *gbox, float4 *gbox_ref, float4 *groups, float4 *fit, const float *lo, const float *hi,
                                const int *child, const long long *first, const int *count, const std::vector<int64_t> &levels, float pad,
                                cudaStream_t stream);
-// Leaf references (drd::kLeafTriF4 float4 each) from the triangle ids in leaf order.
+// Leaf references (drd::kLeafTriF4 float4 each, all first halves before all second ones) from the
+// triangle ids in leaf order.
 cudaError_t launch_leaf_tris(float4 *dst, const int *refs, const float4 *tris, long long n_refs, cudaStream_t stream);
 // Group records (drd::kRecordF4 float4 each) of a scene from its nodes and refitted planes, boxes
 // widened by `pad`; and their copy into a batch arena at group `group_off`, leaf reference `leaf_off`.

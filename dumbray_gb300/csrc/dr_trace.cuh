@@ -210,7 +210,7 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ty
             h.tri = -1;
             h.t = FLT_MAX;
             if (key != kNoHit) {
-                h.tri = leaf_tri_id(S.leaf_tris, (int)(key & 0xFFFFFFFFull));
+                h.tri = leaf_tri_id(S.leaf_tris, S.leaf_half, (int)(key & 0xFFFFFFFFull));
                 h.t = __uint_as_float((unsigned)(key >> 32));
                 h.p = xadd(f3of(ws.o[lane]), xmul(f3of(ws.d[lane]), h.t));
             }
@@ -319,7 +319,7 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ty
                     const int pos = task.y + t;
                     const float4 o = ws.o[task.x], d = ws.d[task.x];
                     float dist;
-                    if (tri_cast(S.leaf_tris, pos, f3of(o), f3of(d), clip, __float_as_int(o.w), dist))
+                    if (tri_cast(S.leaf_tris, S.leaf_half, pos, f3of(o), f3of(d), clip, __float_as_int(o.w), dist))
                         atomicMin(&ws.key[task.x], ((unsigned long long)__float_as_uint(dist) << 32) | (unsigned)pos);
                 }
                 owned += __popc(begins);
