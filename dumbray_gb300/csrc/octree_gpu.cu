@@ -133,9 +133,26 @@ __global__ void __launch_bounds__(32 * kStageWarps) k_split_points(const float *
 // Same call, scenes of the displaced icosphere, physical padding, split 4: with these three kernels
 // (sums, masks, lists) 82k triangles 22.2 -> 18.6 ms, 1.31M triangles 352 -> 297 ms.
 //
+// overlaps() as far as no clipping is needed: the axes in its order (z, x, y), each compared with the
+// whole triangle while the ones before left it whole, and the last one needs no clipped vertices at all.
+// 0 / 1 = its result, 2 = it has to clip.  (Comparisons only: the same result, NaN included, since a
+// triangle with a NaN vertex is left to it.)
+__device__ __forceinline__ int overlaps_plain(const Bx &b, const T3 &t) {
+    const float zl = fminf(fminf(t.a.z, t.b.z), t.c.z), zh = fmaxf(fmaxf(t.a.z, t.b.z), t.c.z);
+    const float xl = fminf(fminf(t.a.x, t.b.x), t.c.x), xh = fmaxf(fmaxf(t.a.x, t.b.x), t.c.x);
+    const float yl = fminf(fminf(t.a.y, t.b.y), t.c.y), yh = fmaxf(fmaxf(t.a.y, t.b.y), t.c.y);
+    const float s = t.a.x + t.a.y + t.a.z + t.b.x + t.b.y + t.b.z + t.c.x + t.c.y + t.c.z;
+    if (s != s) return 2;
+    if (zh < b.lo.z || zl > b.hi.z) return 0;
+    if (!(zl > b.lo.z && zh <= b.hi.z)) return 2;
+    if (xh < b.lo.x || xl > b.hi.x) return 0;
+    if (!(xl > b.lo.x && xh <= b.hi.x)) return 2;
+    return yh < b.lo.y || yl > b.hi.y ? 0 : 1;
+}
+
 // Octant overlap of every reference: a thread per (reference, octant), the mask byte from a ballot.
 // (One thread per reference took its eight tests one after another, each as long as the longest of the
-// warp's.)
+// warp's.  Gathering a block's clipped pairs before clipping them was slower than both.)
 __global__ void k_masks(const float *xyz, const int *refs, const int *owner, const int *off, const float *sub, int nr, int depth,
                         int max_depth, int split_n, unsigned char *mask) {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -160,6 +177,7 @@ __host__ __device__ __forceinline__ Sums operator+(Sums a, Sums b) {
 }
 
 // splittingMakesSence (Octree.impl.cuh:437-475): one warp per node.
+constexpr int kDecideLoads = 8;
 __global__ void k_decide(const unsigned char *mask, const int *off, int nl, int depth, int max_depth, int split_n, int *occ,
                          int *does_split, Sums *sums) {
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -168,9 +186,21 @@ __global__ void k_decide(const unsigned char *mask, const int *off, int nl, int 
     const bool can = splittable(off, k, depth, max_depth, split_n);
     int c[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (can)
-        for (int r = off[k] + lane; r < off[k + 1]; r += 32) {
-            const unsigned m = mask[r];
-            for (int i = 0; i < 8; i++) c[i] += (m >> i) & 1u;
+        for (int base = off[k] + lane; base < off[k + 1]; base += 32 * kDecideLoads) {   // several loads in flight
+            unsigned m[kDecideLoads];
+#pragma unroll
+            for (int q = 0; q < kDecideLoads; q++) m[q] = base + 32 * q < off[k + 1] ? mask[base + 32 * q] : 0u;
+            // bits to byte counters: 4 octants a word
+            unsigned lo = 0, hi = 0;
+#pragma unroll
+            for (int q = 0; q < kDecideLoads; q++) {
+                lo += ((m[q] & 0xFu) * 0x00204081u) & 0x01010101u;
+                hi += ((m[q] >> 4) * 0x00204081u) & 0x01010101u;
+            }
+            for (int i = 0; i < 4; i++) {
+                c[i] += (lo >> (8 * i)) & 0xFF;
+                c[4 + i] += (hi >> (8 * i)) & 0xFF;
+            }
         }
     for (int i = 0; i < 8; i++)
         for (int s = 16; s > 0; s >>= 1) c[i] += __shfl_xor_sync(0xFFFFFFFFu, c[i], s);
@@ -423,36 +453,80 @@ __global__ void __launch_bounds__(32 * kScatterWarps) k_scatter(const int *refs,
 
 inline unsigned blocks(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
+// One allocation that a build's buffers start out from: the levels of a tree would otherwise allocate and
+// free some hundred times (82k triangles, same call: 9.66 -> 7.49 ms a scene, with the decide kernel's
+// loads in flight; 1.31M triangles 109 -> 104 ms).
+struct Slab {
+    char *p = nullptr;
+    size_t bytes = 0, used = 0;
+    explicit Slab(size_t want) {
+        if (want == 0) return;
+        if (cudaMalloc((void **)&p, want) == cudaSuccess) bytes = want;
+        else {
+            p = nullptr;
+            (void)cudaGetLastError();   // the buffers then allocate by themselves
+        }
+    }
+    Slab(const Slab &) = delete;
+    Slab &operator=(const Slab &) = delete;
+    ~Slab() { cudaFree(p); }
+    void *take(size_t want) {
+        want = (want + 255) & ~size_t(255);
+        if (want > bytes - used) return nullptr;
+        void *q = p + used;
+        used += want;
+        return q;
+    }
+};
+
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
+    bool owned = false;
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
-    ~DevBuf() { cudaFree(p); }
+    ~DevBuf() {
+        if (owned) cudaFree(p);
+    }
+    // At least `count` elements, contents undefined.  With a slab the first allocation comes from it, of
+    // `guess` elements if that is more; growing takes half as much again as needed.
+    template <class T>
+    T *get(size_t count, Slab *slab = nullptr, size_t guess = 0) {
+        const size_t need = std::max<size_t>(count, 1) * sizeof(T);
+        if (need > bytes) {
+            const size_t take = bytes ? need + need / 2 : need;
+            if (owned) cudaFree(p);
+            p = nullptr;
+            owned = false;
+            if (!bytes && slab) {
+                const size_t want = std::max(need, guess * sizeof(T));
+                p = slab->take(want);
+                bytes = p ? want : 0;
+            }
+            if (!p) {
+                bytes = 0;
+                if (cudaMalloc(&p, take) != cudaSuccess) {
+                    p = nullptr;
+                    return nullptr;
+                }
+                owned = true;
+                bytes = take;
+            }
+        }
+        return (T *)p;
+    }
     void *release() {
         void *q = p;
         p = nullptr;
         bytes = 0;
+        owned = false;
         return q;
     }
     void swap(DevBuf &o) {
         std::swap(p, o.p);
         std::swap(bytes, o.bytes);
-    }
-    template <class T>
-    T *get(size_t count) {
-        const size_t need = std::max<size_t>(count, 1) * sizeof(T);
-        if (need > bytes) {
-            // half as much again, so that the growing levels do not allocate each time
-            const size_t take = bytes ? need + need / 2 : need;
-            cudaFree(p);
-            p = nullptr;
-            bytes = 0;
-            if (cudaMalloc(&p, take) != cudaSuccess) return nullptr;
-            bytes = take;
-        }
-        return (T *)p;
+        std::swap(owned, o.owned);
     }
 };
 
@@ -486,9 +560,14 @@ bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, Flat
         }
     }
 
+    // references of a level: 4 a triangle with the physical padding, up to 10 with the reference's; nodes:
+    // about one a triangle.  What a level needs beyond that it allocates; past 4M triangles (2.6 GB here)
+    // the allocations no longer show and the guesses would only hold memory.
+    const size_t few = (size_t)n + 64, many = 4 * (size_t)n + 1024;
+    Slab slab(n <= (4 << 20) ? many * 49 + few * 284 + 160 * few : 0);
     DevBuf b_xyz, b_refs, b_next, b_owner, b_centre, b_bounds, b_mask, b_off, b_noff, b_sub, b_occ, b_split, b_lbox, b_fc, b_sums, b_tot;
     float *d_xyz = b_xyz.get<float>(9 * (size_t)n);
-    int *d_refs = b_refs.get<int>((size_t)n);
+    int *d_refs = b_refs.get<int>((size_t)n, &slab, many);
     if (!d_xyz || !d_refs) { err = "device allocation failed"; return false; }
     cudaMemcpy(d_xyz, xyz, 36 * (size_t)n, cudaMemcpyHostToDevice);
     k_iota<<<blocks(n, 256), 256>>>(d_refs, (int)n);
@@ -506,8 +585,8 @@ bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, Flat
     {
         const float b[6] = {root.lo.x, root.lo.y, root.lo.z, root.hi.x, root.hi.y, root.hi.z};
         const int off[2] = {0, (int)n};
-        float *d_box = levels[0]->box.get<float>(6);
-        int *d_off = b_off.get<int>(2);
+        float *d_box = levels[0]->box.get<float>(6, &slab);
+        int *d_off = b_off.get<int>(2, &slab, few);
         if (!d_box || !d_off) { err = "device allocation failed"; return false; }
         cudaMemcpy(d_box, b, sizeof(b), cudaMemcpyHostToDevice);
         cudaMemcpy(d_off, off, sizeof(off), cudaMemcpyHostToDevice);
@@ -520,18 +599,18 @@ bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, Flat
         const int chunks = (nl + kScan - 1) / kScan;
         const int *d_off = (const int *)b_off.p;
         float *d_box = (float *)lv.box.p;
-        int *d_owner = b_owner.get<int>(nr);
-        float *d_centre = b_centre.get<float>(3 * (size_t)nr);
-        float *d_sub = b_sub.get<float>(48 * (size_t)nl);
-        unsigned char *d_mask = b_mask.get<unsigned char>(nr);
-        int *d_occ = b_occ.get<int>(8 * (size_t)nl);
-        int *d_split = b_split.get<int>(nl);
-        float *d_bounds = b_bounds.get<float>(6 * (size_t)nr);
-        float *d_lbox = b_lbox.get<float>(6 * (size_t)nl);
-        Sums *d_sums = b_sums.get<Sums>(nl), *d_tot = b_tot.get<Sums>(chunks + 1);
-        int *d_fc = b_fc.get<int>(nl);
-        int *d_child = lv.child.get<int>(nl), *d_count = lv.count.get<int>(nl);
-        long long *d_first = lv.first.get<long long>(nl);
+        int *d_owner = b_owner.get<int>(nr, &slab, many);
+        float *d_centre = b_centre.get<float>(3 * (size_t)nr, &slab, 3 * many);
+        float *d_sub = b_sub.get<float>(48 * (size_t)nl, &slab, 48 * few);
+        unsigned char *d_mask = b_mask.get<unsigned char>(nr, &slab, many);
+        int *d_occ = b_occ.get<int>(8 * (size_t)nl, &slab, 8 * few);
+        int *d_split = b_split.get<int>(nl, &slab, few);
+        float *d_bounds = b_bounds.get<float>(6 * (size_t)nr, &slab, 6 * many);
+        float *d_lbox = b_lbox.get<float>(6 * (size_t)nl, &slab, 6 * few);
+        Sums *d_sums = b_sums.get<Sums>(nl, &slab, few), *d_tot = b_tot.get<Sums>(chunks + 1, &slab, few / kScan + 2);
+        int *d_fc = b_fc.get<int>(nl, &slab, few);
+        int *d_child = lv.child.get<int>(nl, &slab), *d_count = lv.count.get<int>(nl, &slab);
+        long long *d_first = lv.first.get<long long>(nl, &slab);
         if (!d_owner || !d_centre || !d_sub || !d_mask || !d_occ || !d_split || !d_bounds || !d_lbox || !d_sums || !d_tot || !d_fc ||
             !d_child || !d_count || !d_first) {
             err = "device allocation failed";
@@ -568,10 +647,10 @@ bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, Flat
         next->base = next_base;
         lv.leaf_base = leaf_total;
         lv.leaf_refs = total.leaf_refs;
-        float *d_nbox = next->box.get<float>(6 * (size_t)next->nodes);
-        int *d_noff = b_noff.get<int>((size_t)next->nodes + 1);
-        int *d_next = b_next.get<int>((size_t)total.child_refs);
-        int *d_leaf = lv.leaf.get<int>((size_t)total.leaf_refs);
+        float *d_nbox = next->box.get<float>(6 * (size_t)next->nodes, &slab);
+        int *d_noff = b_noff.get<int>((size_t)next->nodes + 1, &slab, few);
+        int *d_next = b_next.get<int>((size_t)total.child_refs, &slab, many);
+        int *d_leaf = lv.leaf.get<int>((size_t)total.leaf_refs, &slab);
         if (!d_nbox || !d_noff || !d_next || !d_leaf) { err = "device allocation failed"; return false; }
         k_emit<<<blocks(nl, 128), 128>>>(d_sums, d_tot, d_off, d_split, d_occ, d_sub, d_lbox, nl, leaf_total, next_base, d_box, d_child,
                                          d_fc, d_first, d_count, d_noff, d_nbox);
