@@ -132,24 +132,6 @@ __global__ void __launch_bounds__(32 * kStageWarps) k_split_points(const float *
 
 // Same call, scenes of the displaced icosphere, physical padding, split 4: with these three kernels
 // (sums, masks, lists) 82k triangles 22.2 -> 18.6 ms, 1.31M triangles 352 -> 297 ms.
-//
-// overlaps() as far as no clipping is needed: the axes in its order (z, x, y), each compared with the
-// whole triangle while the ones before left it whole, and the last one needs no clipped vertices at all.
-// 0 / 1 = its result, 2 = it has to clip.  (Comparisons only: the same result, NaN included, since a
-// triangle with a NaN vertex is left to it.)
-__device__ __forceinline__ int overlaps_plain(const Bx &b, const T3 &t) {
-    const float zl = fminf(fminf(t.a.z, t.b.z), t.c.z), zh = fmaxf(fmaxf(t.a.z, t.b.z), t.c.z);
-    const float xl = fminf(fminf(t.a.x, t.b.x), t.c.x), xh = fmaxf(fmaxf(t.a.x, t.b.x), t.c.x);
-    const float yl = fminf(fminf(t.a.y, t.b.y), t.c.y), yh = fmaxf(fmaxf(t.a.y, t.b.y), t.c.y);
-    const float s = t.a.x + t.a.y + t.a.z + t.b.x + t.b.y + t.b.z + t.c.x + t.c.y + t.c.z;
-    if (s != s) return 2;
-    if (zh < b.lo.z || zl > b.hi.z) return 0;
-    if (!(zl > b.lo.z && zh <= b.hi.z)) return 2;
-    if (xh < b.lo.x || xl > b.hi.x) return 0;
-    if (!(xl > b.lo.x && xh <= b.hi.x)) return 2;
-    return yh < b.lo.y || yl > b.hi.y ? 0 : 1;
-}
-
 // Octant overlap of every reference: a thread per (reference, octant), the mask byte from a ballot.
 // (One thread per reference took its eight tests one after another, each as long as the longest of the
 // warp's.  Gathering a block's clipped pairs before clipping them was slower than both.)
