@@ -1070,88 +1070,29 @@ struct ShadowPhysSource {
     }
 };
 
-// A block's sums of the gradients it meets most: two-way hashed slots by triangle, claimed by the first
-// triangle that wants one and added to the global array once at the end; a triangle that finds both its
-// slots taken adds to the global array at once.  Large triangles collect most of a frame's gradient
-// (half of all path vertices lie on a room's 12 wall triangles), and their sums were one atomic after
-// another on the same 36 addresses.  1M paths a wave in the room: 0.62-1.17 -> 0.11-0.28 ms a bounce;
-// the whole step (512^2, 16 spp, depth 5, image and gradients) 69.5 -> 60.1 ms in one call.
-constexpr int kGradBits = 9;
-struct GradCache {
-    int tag[1 << kGradBits];             // triangle, -1 = free
-    float sum[3][1 << kGradBits];
-};
-__device__ __forceinline__ void grad_add(float *g, float r, float gg, float b) {
-    if (r != 0.0f) atomicAdd(g, r);
-    if (gg != 0.0f) atomicAdd(g + 1, gg);
-    if (b != 0.0f) atomicAdd(g + 2, b);
-}
-__device__ __forceinline__ void grad_clear(GradCache &c) {
-    for (int k = threadIdx.x; k < 1 << kGradBits; k += blockDim.x) {
-        c.tag[k] = -1;
-        c.sum[0][k] = c.sum[1][k] = c.sum[2][k] = 0.0f;
-    }
-}
-__device__ __forceinline__ void grad_add(GradCache &c, float *grad, int tri, float r, float gg, float b) {
-    const unsigned h = ((unsigned)tri * 0x9E3779B1u) >> (32 - kGradBits);
-#pragma unroll
-    for (unsigned way = 0; way < 2; way++) {
-        const unsigned k = h ^ way;
-        int t = *((volatile int *)&c.tag[k]);
-        if (t == -1) {
-            t = atomicCAS(&c.tag[k], -1, tri);
-            if (t == -1) t = tri;
-        }
-        if (t != tri) continue;
-        if (r != 0.0f) atomicAdd(&c.sum[0][k], r);
-        if (gg != 0.0f) atomicAdd(&c.sum[1][k], gg);
-        if (b != 0.0f) atomicAdd(&c.sum[2][k], b);
-        return;
-    }
-    grad_add(grad + 3 * (size_t)tri, r, gg, b);
-}
-__device__ __forceinline__ void grad_flush(const GradCache &c, float *grad) {
-    for (int k = threadIdx.x; k < 1 << kGradBits; k += blockDim.x)
-        if (c.tag[k] >= 0) grad_add(grad + 3 * (size_t)c.tag[k], c.sum[0][k], c.sum[1][k], c.sum[2][k]);
-}
-
 // Adjoint pass: gradients of the visible NEE contributions of bounce b (k_shadow_phys<ADJ> marks a
 // visible record with s2.x = 1; k_shade_phys writes s2 = {0, 0, 0, tri}), scattered here rather
 // than in the traversal kernel, whose registers then stay the traversal's.  The adjoint is a single
 // render job's, never a batch's.
 __global__ void __launch_bounds__(256) k_adj_shadow(WaveArgs A, int b) {
     const int n = *((volatile int *)&A.ctrl->shadow_count[b]);
-    if ((int)(blockIdx.x * blockDim.x) >= n) return;
-    __shared__ GradCache albedo, emission;
-    grad_clear(albedo);
-    grad_clear(emission);
-    __syncthreads();
-    const Item &I = A.inl;
     for (int i = (int)(blockIdx.x * blockDim.x + threadIdx.x); i < n; i += (int)(gridDim.x * blockDim.x)) {
         if (A.sq.s2[i].x == 0.0f) continue;
         const float4 s4 = A.sq.s4[i];
+        const c3 c = mkc(s4.x, s4.y, s4.z);
+        const Item &I = A.inl;
         const float4 s3 = A.sq.s3[i];
-        const int *pre = A.prefix + (size_t)__float_as_int(s3.x) * kAdjDepth;
-        const int vtx = __float_as_int(s3.y);
+        const int path = __float_as_int(s3.x), vtx = __float_as_int(s3.y);
         const int light_tri = __float_as_int(A.sq.s1[i].w);
         const c3 delta = pixel_adjoint(I, __float_as_int(A.sq.s0[i].w));
-        const float gr = delta.r * s4.x, gg = delta.g * s4.y, gb = delta.b * s4.z;
         const float *lep = I.S.emission + 3 * (size_t)light_tri;
         const float lr = __ldg(lep), lg = __ldg(lep + 1), lb = __ldg(lep + 2);
-        grad_add(emission, I.grad_emission, light_tri, lr > 0.0f && delta.r != 0.0f ? gr / lr : 0.0f,
-                 lg > 0.0f && delta.g != 0.0f ? gg / lg : 0.0f, lb > 0.0f && delta.b != 0.0f ? gb / lb : 0.0f);
-        if (gr == 0.0f && gg == 0.0f && gb == 0.0f) continue;
-        for (int j = 0; j <= vtx; j++) {   // as scatter_albedo
-            const int k = pre[j];
-            const float *a = I.S.albedo + 3 * (size_t)k;
-            const float ar = __ldg(a), ag = __ldg(a + 1), ab = __ldg(a + 2);
-            grad_add(albedo, I.grad_albedo, k, ar > 1e-8f ? gr / ar : 0.0f, ag > 1e-8f ? gg / ag : 0.0f,
-                     ab > 1e-8f ? gb / ab : 0.0f);
-        }
+        float *g = I.grad_emission + 3 * (size_t)light_tri;
+        if (lr > 0.0f && delta.r != 0.0f) atomicAdd(g, delta.r * c.r / lr);
+        if (lg > 0.0f && delta.g != 0.0f) atomicAdd(g + 1, delta.g * c.g / lg);
+        if (lb > 0.0f && delta.b != 0.0f) atomicAdd(g + 2, delta.b * c.b / lb);
+        scatter_albedo(I, A.prefix + (size_t)path * kAdjDepth, vtx, delta, c);
     }
-    __syncthreads();
-    grad_flush(albedo, I.grad_albedo);
-    grad_flush(emission, I.grad_emission);
 }
 
 // Physical visibility: closest hit from the shading point toward the sampled light point
@@ -1543,7 +1484,7 @@ static void launch_wave_t(const WaveDesc &W, const WaveArgs &A, cudaStream_t str
             }
         } else if (!MULTI && W.adjoint) {
             k_shadow_phys<false, false, true, TT, TB><<<tgrid, TT, 0, stream>>>(A, b);
-            k_adj_shadow<<<sm_count() * 4, 256, 0, stream>>>(A, b);
+            k_adj_shadow<<<sm_count() * 8, 256, 0, stream>>>(A, b);
             nl++;
         } else {
             if (count) k_shadow_phys<true, MULTI, false, TT, TB><<<tgrid, TT, 0, stream>>>(A, b);
