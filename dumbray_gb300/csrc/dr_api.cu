@@ -148,6 +148,8 @@ struct dr_renderer {
     drk::Profiler prof;
     unsigned long long *counters = nullptr;
     bool counting = false;
+    float4 *grads = nullptr;        // adjoint: gradient sums of a call, by triangle
+    long long grad_records = 0;
     int *prefix = nullptr;          // adjoint: per-path vertex triangles
     int prefix_paths = 0;
     // Concurrent wave pipelines of dr_render_blocks: the renderer's own scratch on the caller's
@@ -170,6 +172,7 @@ struct dr_renderer {
 
     ~dr_renderer() {
         cudaFree(counters);
+        cudaFree(grads);
         cudaFree(prefix);
         for (int k = 0; k < 2; k++) {
             for (int j = 0; j < 3; j++) cudaFree(q[k][j]);
@@ -1102,8 +1105,6 @@ dr_status dr_render_adjoint(dr_renderer *r, const dr_scene *sc, const dr_camera 
     drk::Item &I = W.inl;
     I.fb = nullptr;
     I.dl_dfb = dl_dfb;
-    I.grad_albedo = grad_albedo;
-    I.grad_emission = grad_emission;
     const long long cap = 1LL << 20;  // paths per adjoint wave: bounds each lane's prefix buffer to ~280 MB
     const long long total = (long long)I.n_slots * I.spp;
     const long long wave = lane_wave(total, wave_size(r, 1, cap), r->lanes);
@@ -1117,13 +1118,30 @@ dr_status dr_render_adjoint(dr_renderer *r, const dr_scene *sc, const dr_camera 
     if (e != cudaSuccess) return cuda_fail(e, "dr_render_adjoint: prefix buffer");
     st = ensure_accum(r, (size_t)I.n_slots);
     if (st != DR_OK) return st;
+    const long long n = I.S.n_tris;
+    if (r->grad_records < 2 * n) {
+        cudaFree(r->grads);
+        r->grads = nullptr;
+        r->grad_records = 0;
+        e = cudaMalloc((void **)&r->grads, sizeof(float4) * 2 * (size_t)n);
+        if (e != cudaSuccess) return cuda_fail(e, "dr_render_adjoint: gradient sums");
+        r->grad_records = 2 * n;
+    }
+    e = drk::load_adjoint_kernels(r->shape);
+    if (e == cudaSuccess) e = cudaMemsetAsync(r->grads, 0, sizeof(float4) * 2 * (size_t)n, stream);
+    if (e != cudaSuccess) return cuda_fail(e, "dr_render_adjoint: gradient sums");
+    I.grad_albedo = r->grads;
+    I.grad_emission = r->grads + n;
     W.items = nullptr;
     W.n_items = 1;
     W.mode = I.mode;
     W.max_bounces = I.max_bounces;
     W.adjoint = true;
     wave_buffers(r, W);
-    return run_waves(r, W, total, wave, I.n_slots, stream, &r->prof, false, false, L);
+    st = run_waves(r, W, total, wave, I.n_slots, stream, &r->prof, false, false, L);
+    if (st != DR_OK) return st;
+    e = drk::add_gradients(r->grads, (int)n, grad_albedo, grad_emission, stream);
+    return e == cudaSuccess ? DR_OK : cuda_fail(e, "dr_render_adjoint: gradient sums");
 } catch (...) {
     return dr_internal_exception("dr_render_adjoint");
 }

@@ -36,8 +36,8 @@ struct Item {
     float *fb;                   // block-major float4 frame buffer
     float inv_spp, blend;
     const float *dl_dfb;         // adjoint: dL/dI, block-major float4 (null outside the adjoint pass)
-    float *grad_albedo;          // adjoint: dL/d albedo, float[n][3]
-    float *grad_emission;        // adjoint: dL/d emission, float[n][3]
+    float4 *grad_albedo;         // adjoint: sums of this call's dL/d albedo by triangle, w unused
+    float4 *grad_emission;       // adjoint: sums of this call's dL/d emission
 };
 
 // One wave: paths [wave_begin, wave_begin + wave_count) of the path space of all jobs.
@@ -93,6 +93,9 @@ class Profiler {
     cudaEvent_t base_ = nullptr;
 };
 
+cudaError_t load_adjoint_kernels(int shape);   // shape: see WaveDesc
+// Adds the gradient sums of an adjoint pass (n albedo records, then n emission records) to float[n][3] arrays.
+cudaError_t add_gradients(const float4 *sums, int n, float *albedo, float *emission, cudaStream_t stream);
 size_t ctrl_bytes();
 // Per-bounce queue counts of the wave last run on control block `ctrl`: rays[b] = extension rays
 // traced at bounce b, shadows[b] = shadow / photon records queued at bounce b (b < n <= kMaxBounceSlots).
