@@ -177,8 +177,10 @@ __host__ __device__ constexpr int steps_per_round(bool physical) { return physic
 
 // ---------------------------------------------------------------------------------------------
 // dr_cast: warp w of the grid traces rays [w c, (w + 1) c), then the same of every next grid's worth
-// (c = 32, or fewer when the rays do not fill the lanes).  Neighbouring rays stay together, a warp
-// refills its lanes until its last chunk, and no counter has to be cleared or kept between calls.
+// (c = 32, or fewer when the rays do not fill the lanes).  A warp refills its lanes until its last chunk,
+// and no counter has to be cleared or kept between calls.  SPREAD: the rays are taken in pairs from 16
+// parts of the batch in turn (see neighbours_alike).
+template <bool SPREAD>
 struct BatchSource {
     static constexpr float kOccludeBelow = 0.0f;
     const float *o, *d;
@@ -189,6 +191,12 @@ struct BatchSource {
     unsigned at;          // the warp's next chunk
     bool cull;
     const Scene *scene0;  // unused: single-scene source
+    unsigned row;         // SPREAD: pairs in a part
+    __device__ __forceinline__ int entry(int k) {
+        if (!SPREAD) return k;
+        const unsigned g = (unsigned)k >> 1;
+        return g < row << 4 ? (int)((((g & 15u) * row + (g >> 4)) << 1) + (k & 1)) : k;   // the last n % 32 in order
+    }
     __device__ __forceinline__ bool next(int &b, int &e) {
         if (at >= (unsigned)n) return false;
         b = (int)at;
@@ -222,15 +230,32 @@ constexpr int kCastThreads = 64;
 // 64 registers, 32 warps per SM; the counting traversal needs 80.
 constexpr int cast_blocks_per_sm(bool count) { return count ? 12 : 16; }
 
-template <bool COUNT>
+// Whether most rays of a batch go nearly the way of the next one (within 11 degrees): 32 pairs looked at,
+// a lane each, the same for every warp; n >= 64.  Neighbours that see one silhouette are all slow (a
+// grazing ray takes up to 250 times the mean), and the warp that got 32 of them ended a launch long after
+// the others.  Spread over the warps, same call: 1080p primary casts 1161 -> 736 us, 0.5M 801 -> 458,
+// 8.3M 2.38 -> 1.91 ms.  Rays in random order are spread already, and lose 1-4% if they are taken in pairs
+// from far apart; so both kernels are launched and one of them leaves at once, which costs them 9 of 275 us
+// at 0.5M rays, 0-1% from 1M on.  One kernel with the order as a variable, or with both loops, cost the
+// random order 1-5% in registers, and the pairs' loop out of line made that one 5% slower.
+__device__ __forceinline__ bool neighbours_alike(const float *__restrict__ d, int n) {
+    const float *a = d + 3 * ((size_t)lane_id() * (unsigned)(n >> 5));
+    const float ax = __ldg(a), ay = __ldg(a + 1), az = __ldg(a + 2), bx = __ldg(a + 3), by = __ldg(a + 4), bz = __ldg(a + 5);
+    const float ab = ax * bx + ay * by + az * bz, aa = ax * ax + ay * ay + az * az, bb = bx * bx + by * by + bz * bz;
+    return __popc(__ballot_sync(0xFFFFFFFFu, ab > 0.0f && ab * ab > 0.96f * aa * bb)) > 16;
+}
+
+// two_orders: this launch is one of two, for the batches its order suits.
+template <bool COUNT, bool SPREAD>
 __global__ void __launch_bounds__(kCastThreads, cast_blocks_per_sm(COUNT))
     k_cast(Scene S, const float *__restrict__ o, const float *__restrict__ d, const int *__restrict__ ignore, int n, int clip,
-           int *__restrict__ hit_tri, float *__restrict__ hit_t, int *__restrict__ nbox, int *__restrict__ ntri) {
+           int *__restrict__ hit_tri, float *__restrict__ hit_t, int *__restrict__ nbox, int *__restrict__ ntri, int two_orders) {
+    if (two_orders && neighbours_alike(d, n) != SPREAD) return;
     typename StackOf<COUNT>::type stack[kStack];
     __shared__ WarpSlots slots[kCastThreads / 32];
     const int width = warp_width(n, grid_warps());
     const unsigned warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    BatchSource src{o, d, ignore, hit_tri, COUNT ? nbox : nullptr, COUNT ? ntri : nullptr, hit_t, n, width, warp * width, clip != 0, &S};
+    BatchSource<SPREAD> src{o, d, ignore, hit_tri, COUNT ? nbox : nullptr, COUNT ? ntri : nullptr, hit_t, n, width, warp * width, clip != 0, &S, (unsigned)n >> 5};
     trace_persistent<COUNT, false>(S, src, stack, slots[threadIdx.x >> 5], width, steps_per_round(S.front_only != 0));
 }
 
@@ -442,6 +467,7 @@ struct TraceSource {
     int n, chunk;
     long long rays, nb, nt;
     __device__ __forceinline__ bool next(int &b, int &e) { return fetch_chunk(fetch, n, chunk, b, e); }
+    __device__ __forceinline__ int entry(int k) { return k; }
     __device__ __forceinline__ bool load(int i, f3 &o, f3 &d, int &ign, int &job) {
         float4 p0 = Q.p0[i], p1 = Q.p1[i];
         int4 p3 = Q.p3[i];
@@ -673,6 +699,7 @@ struct RefPhotonSource {
     int n, chunk;
     long long rays, nb, nt;
     __device__ __forceinline__ bool next(int &b, int &e) { return fetch_chunk(fetch, n, chunk, b, e); }
+    __device__ __forceinline__ int entry(int k) { return k; }
     __device__ __forceinline__ bool load(int i, f3 &o, f3 &d, int &ign, int &job) {
         o = f3of(sq.s0[i]);
         d = f3of(sq.s1[i]);
@@ -753,6 +780,7 @@ struct RefPhotonChainSource {
     int n, chunk;
     long long rays, nb, nt;
     __device__ __forceinline__ bool next(int &b, int &e) { return fetch_chunk(fetch, n, chunk, b, e); }
+    __device__ __forceinline__ int entry(int k) { return k; }
     __device__ __forceinline__ bool load(int i, f3 &o, f3 &d, int &ign, int &job) {
         const int j = kept ? kept[i] : i;
         const int w = __float_as_int(sq.s3[j].w);   // negative: a roomy wave's photon, not shaded yet
@@ -1046,6 +1074,7 @@ struct ShadowPhysSource {
     int n, chunk;
     long long rays, nb, nt;
     __device__ __forceinline__ bool next(int &b, int &e) { return fetch_chunk(fetch, n, chunk, b, e); }
+    __device__ __forceinline__ int entry(int k) { return k; }
     __device__ __forceinline__ bool load(int i, f3 &o, f3 &d, int &ign, int &job) {
         o = f3of(sq.s0[i]);
         d = f3of(sq.s1[i]);
@@ -1319,11 +1348,16 @@ cudaError_t launch_cast(const Scene &S, const float *o, const float *d, const in
     // one warp per ray until the resident warps are used up
     const int blocks = (int)std::min<long long>((n + kCastThreads / 32 - 1) / (kCastThreads / 32),
                                                 (long long)sm_count() * cast_blocks_per_sm(nbox || ntri));
-    if (nbox || ntri)
-        k_cast<true><<<blocks, kCastThreads, 0, stream>>>(S, o, d, ignore, n, clip, hit_tri, hit_t, nbox, ntri);
-    else
-        k_cast<false><<<blocks, kCastThreads, 0, stream>>>(S, o, d, ignore, n, clip, hit_tri, hit_t, nullptr, nullptr);
-    if (launches) (*launches)++;
+    const bool two = n >= 32LL * (kCastThreads / 32) * blocks;   // several chunks a warp: see neighbours_alike
+    auto go = [&](auto kernel) { kernel<<<blocks, kCastThreads, 0, stream>>>(S, o, d, ignore, n, clip, hit_tri, hit_t, nbox, ntri, two); };
+    if (nbox || ntri) {
+        go(k_cast<true, false>);
+        if (two) go(k_cast<true, true>);
+    } else {
+        go(k_cast<false, false>);
+        if (two) go(k_cast<false, true>);
+    }
+    if (launches) *launches += two ? 2 : 1;
     return cudaGetLastError();
 }
 

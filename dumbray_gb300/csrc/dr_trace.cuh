@@ -159,6 +159,7 @@ __device__ __forceinline__ int warp_width(int n, int warps) { return max(1, min(
 
 // Source interface:
 //   bool next(int &begin, int &end)           warp-uniform; false when no work is left
+//   int entry(int k)                          the k-th ray to take
 //   bool load(int i, f3 &o, f3 &d, int &ignore, int &job)   false: entry i needs no cast (done)
 //   int job(int i)                            the job of entry i
 //   const Scene &scene(int job)               the scene of a job (MULTI only)
@@ -225,7 +226,7 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ty
                 const int avail = c_end - c_next;
                 const int rank = __popc(want & lt_mask);
                 if (free && rank < avail) {
-                    cur_i = c_next + rank;
+                    cur_i = src.entry(c_next + rank);
                     start = true;
                 }
                 c_next += min(avail, __popc(want));
