@@ -1361,16 +1361,17 @@ cudaError_t launch_cast(const Scene &S, const float *o, const float *d, const in
     return cudaGetLastError();
 }
 
-// The call's gradient sums, two arrays of n records one after the other, added to the caller's arrays.
+// The call's gradient sums, two arrays of n records one after the other, added to the caller's arrays:
+// atomically, since renderers on other streams may add other blocks' gradients to the same arrays.
 __global__ void k_add_gradients(const float4 *__restrict__ sums, int n, float *albedo, float *emission) {
     for (int k = (int)(blockIdx.x * blockDim.x + threadIdx.x); k < n; k += (int)(gridDim.x * blockDim.x))
 #pragma unroll
         for (int a = 0; a < 2; a++) {
             const float4 v = sums[a ? (size_t)n + k : (size_t)k];
             float *g = (a ? emission : albedo) + 3 * (size_t)k;
-            if (v.x != 0.0f) g[0] += v.x;
-            if (v.y != 0.0f) g[1] += v.y;
-            if (v.z != 0.0f) g[2] += v.z;
+            if (v.x != 0.0f) atomicAdd(g, v.x);
+            if (v.y != 0.0f) atomicAdd(g + 1, v.y);
+            if (v.z != 0.0f) atomicAdd(g + 2, v.z);
         }
 }
 cudaError_t add_gradients(const float4 *sums, int n, float *albedo, float *emission, cudaStream_t stream) {

@@ -46,3 +46,22 @@ def test_gradients_add_up_over_blocks(cuda, levels, width, height, depth):
             r.render_adjoint(sc, cam, dl, b, b + 1, params, part[0], part[1])
             want += part.double()
         assert torch.allclose(got.double(), want, rtol=6e-4, atol=6e-8)
+
+
+def test_renderers_on_two_streams_add_to_the_same_arrays(cuda):
+    sc = _scene(3)
+    cam = dr.camera(dr.LENS_PINHOLE, position=(0.0, 0.0, -0.97), angle=60.0)
+    width, height, rounds = 64, 64, 6
+    params = dr.render_params(width, height, dr.MODE_PHYSICAL, samples=(1, 1), max_bounces=2, seed=9)
+    nb = dr.block_count(width, height)
+    dl = dr.new_frame_buffer(width, height, cuda) + 0.5
+    renderers, streams = [dr.Renderer(1 << 14) for _ in range(2)], [torch.cuda.Stream() for _ in range(2)]
+    got, one = torch.zeros((2, sc.n, 3), device=cuda), torch.zeros((2, sc.n, 3), device=cuda)
+    renderers[0].render_adjoint(sc, cam, dl, 0, nb, params, one[0], one[1])
+    torch.cuda.synchronize()
+    for _ in range(rounds):
+        for r, s in zip(renderers, streams):
+            r.render_adjoint(sc, cam, dl, 0, nb, params, got[0], got[1], stream=s)
+    torch.cuda.synchronize()
+    # 4,096 paths of up to 3 terms a component: either sum is within 12,288 * 2^-24 = 7.4e-4 of its value
+    assert torch.allclose(got.double(), 2 * rounds * one.double(), rtol=1.5e-3, atol=1e-6)
