@@ -358,9 +358,12 @@ struct RaySlopes {
 };
 // The direction is scaled to a largest component in [1, 2) (a power of two: exact), so only origins
 // beyond 1e24 could take a product out of the float range; such an axis is not tested (near = -max,
-// far = +max).  A component below 2^-40 of the largest is raised to that: over the t range of the
-// scene it moves the ray by less than 2^-39 of reach + |o|, far inside the widening, and 0 * inf does
-// not arise.
+// far = +max).  A component below 2^-40 of the largest is raised to that, so that 0 * inf does not arise.
+// That shears the ray along the component's axis: at parameter t by up to 2^-40 |t|, which in units of the
+// axis' plane distances is |t| itself, far more than the widening when the origin is far away along another
+// axis.  In any box of the scene |t| is at most reach + |o.x| + |o.y| + |o.z| (the scaled direction's largest
+// component is 1 or more; 2^-22 or more if it is denormal), so both offsets of such an axis take twice that
+// and the exact test's kEps (`shear`).
 __device__ __forceinline__ RaySlopes ray_slopes(f3 o, f3 d, float reach) {
     RaySlopes r;
     const float oc[3] = {o.x, o.y, o.z}, dc[3] = {d.x, d.y, d.z};
@@ -368,12 +371,13 @@ __device__ __forceinline__ RaySlopes ray_slopes(f3 o, f3 d, float reach) {
     const unsigned e2 = min(__float_as_uint(dmax) >> 23, 253u);
     const float up = __uint_as_float((254u - e2) << 23), eps2 = 2.0f * kEps * __uint_as_float(e2 << 23);   // t shrinks by `up`
     constexpr float kTiny = 9.094947017729282e-13f;   // 2^-40
+    const float shear = eps2 + (fabsf(o.x) + fabsf(o.y) + fabsf(o.z) + reach) * (e2 == 0u ? 8388608.0f : 2.0f);   // sum as in point_margin
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        const float a = fmaxf(fabsf(dc[k]) * up, kTiny);
+        const float scaled = fabsf(dc[k]) * up, a = fmaxf(scaled, kTiny);
         float inv;
         asm("rcp.approx.f32 %0, %1;" : "=f"(inv) : "f"(dc[k] < 0.0f ? -a : a));   // within an ulp: part of the slack
-        const float oi = oc[k] * inv, e = fabsf(oi) * kRaySlack;
+        const float oi = oc[k] * inv, e = fabsf(oi) * kRaySlack + (scaled < kTiny ? shear : 0.0f);
         const bool ok = fabsf(inv) * (reach + fabsf(oc[k])) < 1e37f;
         const float i = ok ? inv : 0.0f, n = ok ? -oi - e : -FLT_MAX, f = ok ? eps2 + e - oi : FLT_MAX;
         r.inv[k] = pack2(i, i);
