@@ -494,14 +494,17 @@ struct TraceSource {
 // Block shape of the traversal kernels (k_trace, k_shadow_phys, k_shadow_ref): 8 warps, 4 blocks per SM
 // cap registers at 64 (32 warps per SM), which the traversal state fits without spilling.  4 against 3
 // blocks (80 registers), in one call: room 9.40 -> 8.67 ms, 1080p photon render 44.2 -> 42.1 ms, path
-// trace 38.4 -> 35.7 ms, gradients 73.0 -> 70.4 ms.
+// trace 38.4 -> 35.7 ms, gradients 73.0 -> 70.4 ms.  The counting instances hold boxes and counts as well and
+// spill 126 bytes at 64 registers; 3 blocks (80 registers): 256^2 x 4 counted renders 3.04 -> 2.86 ms in the
+// room, 5.83 -> 5.37 ms on 1.31M triangles.  k_shadow_ref<COUNT> loses 2-3% on spotlights there and keeps 4.
 constexpr int kTraceThreads = 256;
 constexpr int kTraceBlocksPerSM = 4;
+constexpr int counted_blocks(bool count, int blocks) { return count ? blocks * 3 / 4 : blocks; }
 
 // Block shapes a renderer can select (dr_renderer_set_block_shape): 0 = 256 x 4, 1 = 128 x 8 per SM
 // (both cap registers at 64); the autotuner times them.
 template <bool COUNT, bool MULTI, int TT = kTraceThreads, int TB = kTraceBlocksPerSM>
-__global__ void __launch_bounds__(TT, TB) k_trace(WaveArgs A, int b) {
+__global__ void __launch_bounds__(TT, counted_blocks(COUNT, TB)) k_trace(WaveArgs A, int b) {
     Ctrl *C = A.ctrl;
     const int n = *((volatile int *)&C->ray_count[b]);
     typename StackOf<COUNT>::type stack[kStack];
@@ -1132,7 +1135,7 @@ __global__ void __launch_bounds__(256) k_adj_shadow(WaveArgs A, int b) {
 // (direction = light point - shading point, so the light is at t = 1), ignoring the shading
 // triangle; visible if nothing but the light triangle is hit before t = 0.999.
 template <bool COUNT, bool MULTI, bool ADJ, int TT = kTraceThreads, int TB = kTraceBlocksPerSM>
-__global__ void __launch_bounds__(TT, TB) k_shadow_phys(WaveArgs A, int b) {
+__global__ void __launch_bounds__(TT, counted_blocks(COUNT, TB)) k_shadow_phys(WaveArgs A, int b) {
     Ctrl *C = A.ctrl;
     const int n = *((volatile int *)&C->shadow_count[b]);
     typename StackOf<COUNT>::type stack[kStack];
@@ -1530,7 +1533,7 @@ static void launch_wave_t(const WaveDesc &W, const WaveArgs &A, cudaStream_t str
     k_camera<MULTI><<<std::min(grid, (W.wave_count + kCameraThreads - 1) / kCameraThreads), kCameraThreads, 0, stream>>>(A);
     P.end(KC_CAMERA, stream);
     nl++;
-    const int tgrid = sm_count() * TB;   // one persistent block per slot
+    const int tgrid = sm_count() * counted_blocks(count, TB);   // one persistent block per slot
     for (int b = 0; b <= W.max_bounces; b++) {
         P.begin(KC_TRACE, stream);
         if (count) k_trace<true, MULTI, TT, TB><<<tgrid, TT, 0, stream>>>(A, b);
