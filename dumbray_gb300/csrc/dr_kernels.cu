@@ -239,12 +239,15 @@ constexpr int cast_blocks_per_sm(bool count) { return count ? 12 : 16; }
 // 8.3M 2.38 -> 1.91 ms.  Rays in random order are spread already, and lose 1-4% if they are taken in pairs
 // from far apart; so both kernels are launched and one of them leaves at once, which costs them 9 of 275 us
 // at 0.5M rays, 0-1% from 1M on.  One kernel with the order as a variable, or with both loops, cost the
-// random order 1-5% in registers, and the pairs' loop out of line made that one 5% slower.
+// random order 1-5% in registers, and the pairs' loop out of line made that one 5% slower.  Each kernel
+// decides by itself, so the operations are explicitly rounded: with two roundings of the same expression a
+// batch at the line would be cast by both kernels or by neither.
 __device__ __forceinline__ bool neighbours_alike(const float *__restrict__ d, int n) {
     const float *a = d + 3 * ((size_t)lane_id() * (unsigned)(n >> 5));
     const float ax = __ldg(a), ay = __ldg(a + 1), az = __ldg(a + 2), bx = __ldg(a + 3), by = __ldg(a + 4), bz = __ldg(a + 5);
-    const float ab = ax * bx + ay * by + az * bz, aa = ax * ax + ay * ay + az * az, bb = bx * bx + by * by + bz * bz;
-    return __popc(__ballot_sync(0xFFFFFFFFu, ab > 0.0f && ab * ab > 0.96f * aa * bb)) > 16;
+    const f3 u = mkf3(ax, ay, az), v = mkf3(bx, by, bz);
+    const float ab = xdot(u, v);
+    return __popc(__ballot_sync(0xFFFFFFFFu, ab > 0.0f && __fmul_rn(ab, ab) > __fmul_rn(__fmul_rn(0.96f, xdot(u, u)), xdot(v, v)))) > 16;
 }
 
 // two_orders: this launch is one of two, for the batches its order suits.
