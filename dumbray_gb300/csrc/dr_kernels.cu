@@ -867,9 +867,16 @@ __device__ __forceinline__ c3 pixel_adjoint(const Item &I, int slot) {
 // addresses, one after another, were a fifth of an adjoint step.  1M paths a wave in the room, the whole step
 // (512^2, 16 spp, depth 5, image and gradients): 65.8 -> 58.4 ms in one call.  Every term is still added
 // to one float32 sum by itself: block sums would be quicker yet (55.5 ms) but keep small terms that the
-// long sums lose, 0.4% on a wall.
-__device__ __forceinline__ void grad_add(float4 *g, float r, float gg, float b) {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g), "f"(r), "f"(gg), "f"(b), "f"(0.0f) : "memory");
+// long sums lose, 0.4% on a wall.  stride 3: straight to the caller's arrays (dr_render_adjoint says when).
+__device__ __forceinline__ void grad_add(float *sums, int stride, int k, float r, float gg, float b) {
+    float *g = sums + (size_t)k * stride;
+    if (stride == 4) {
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g), "f"(r), "f"(gg), "f"(b), "f"(0.0f) : "memory");
+        return;
+    }
+    if (r != 0.0f) atomicAdd(g, r);
+    if (gg != 0.0f) atomicAdd(g + 1, gg);
+    if (b != 0.0f) atomicAdd(g + 2, b);
 }
 // A contribution c (per channel) carrying the albedo factors of path vertices prefix[0..last]:
 // d c / d albedo_k = c / albedo_k for each such vertex (every material scales the throughput, and
@@ -881,7 +888,7 @@ __device__ __forceinline__ void scatter_albedo(const Item &I, const int *pre, in
         int k = pre[j];
         const float *a = I.S.albedo + 3 * (size_t)k;
         float ar = __ldg(a), ag = __ldg(a + 1), ab = __ldg(a + 2);
-        grad_add(I.grad_albedo + k, ar > 1e-8f ? gr / ar : 0.0f, ag > 1e-8f ? gg / ag : 0.0f, ab > 1e-8f ? gb / ab : 0.0f);
+        grad_add(I.grad_albedo, I.grad_stride, k, ar > 1e-8f ? gr / ar : 0.0f, ag > 1e-8f ? gg / ag : 0.0f, ab > 1e-8f ? gb / ab : 0.0f);
     }
 }
 
@@ -957,7 +964,7 @@ __global__ void __launch_bounds__(kShadeThreads, kShadePhysBlocksPerSM) k_shade_
                     c3 c = mkc(thr.r * em.r * w, thr.g * em.g * w, thr.b * em.b * w);
                     if (ADJ) {
                         c3 delta = pixel_adjoint(I, slot);
-                        grad_add(I.grad_emission + tri, delta.r != 0.0f ? delta.r * thr.r * w : 0.0f,
+                        grad_add(I.grad_emission, I.grad_stride, tri, delta.r != 0.0f ? delta.r * thr.r * w : 0.0f,
                                  delta.g != 0.0f ? delta.g * thr.g * w : 0.0f, delta.b != 0.0f ? delta.b * thr.b * w : 0.0f);
                         if (b > 0) scatter_albedo(I, A.prefix + (size_t)path * kAdjDepth, b - 1, delta, c);
                     } else {
@@ -1128,7 +1135,7 @@ __global__ void __launch_bounds__(256) k_adj_shadow(WaveArgs A, int b) {
         const c3 delta = pixel_adjoint(I, __float_as_int(A.sq.s0[i].w));
         const float *lep = I.S.emission + 3 * (size_t)light_tri;
         const float lr = __ldg(lep), lg = __ldg(lep + 1), lb = __ldg(lep + 2);
-        grad_add(I.grad_emission + light_tri, lr > 0.0f && delta.r != 0.0f ? delta.r * c.r / lr : 0.0f,
+        grad_add(I.grad_emission, I.grad_stride, light_tri, lr > 0.0f && delta.r != 0.0f ? delta.r * c.r / lr : 0.0f,
                  lg > 0.0f && delta.g != 0.0f ? delta.g * c.g / lg : 0.0f, lb > 0.0f && delta.b != 0.0f ? delta.b * c.b / lb : 0.0f);
         scatter_albedo(I, A.prefix + (size_t)path * kAdjDepth, vtx, delta, c);
     }

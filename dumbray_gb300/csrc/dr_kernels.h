@@ -36,8 +36,9 @@ struct Item {
     float *fb;                   // block-major float4 frame buffer
     float inv_spp, blend;
     const float *dl_dfb;         // adjoint: dL/dI, block-major float4 (null outside the adjoint pass)
-    float4 *grad_albedo;         // adjoint: sums of this call's dL/d albedo by triangle, w unused
-    float4 *grad_emission;       // adjoint: sums of this call's dL/d emission
+    float *grad_albedo;          // adjoint: dL/d albedo, grad_stride floats a triangle
+    float *grad_emission;        // adjoint: dL/d emission, likewise
+    int grad_stride;             // adjoint: 4 = padded sums of this call (w unused), 3 = the caller's float[n][3]
 };
 
 // One wave: paths [wave_begin, wave_begin + wave_count) of the path space of all jobs.

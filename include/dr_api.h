@@ -366,7 +366,10 @@ dr_status dr_render_blocks(dr_renderer *r, const dr_scene *scene, const dr_camer
  * (device float[n][3] each) for the scene's triangles.  The paths are regenerated from the
  * counter-based random numbers of `params` (same seed / iteration as the forward render), so no
  * path is stored between the passes: memory is the renderer's wave scratch plus one triangle id
- * per path vertex of the paths in flight.  Sampling pdfs (light selection, BSDF, MIS) are treated
+ * per path vertex of the paths in flight, and from some thousand paths a call on gradient sums of 32
+ * bytes per triangle, which the renderer keeps and grows.  A call that is captured into a CUDA graph
+ * adds straight to the gradient arrays instead (the graph must not outlive the renderer, nor a later
+ * call of it with more pixels or a larger wave, whose scratch replaces the captured one).  Sampling pdfs (light selection, BSDF, MIS) are treated
  * as constants, which keeps the gradient estimate unbiased. */
 dr_status dr_render_adjoint(dr_renderer *r, const dr_scene *scene, const dr_camera *camera, const float *dl_dfb_blockmajor,
                             int32_t start_block, int32_t end_block, const dr_render_params *params, float *grad_albedo,
