@@ -767,12 +767,16 @@ dr_status dr_cast_counted(const dr_scene *sc, const float *o, const float *d, co
     return dr_internal_exception("dr_cast_counted");
 }
 
+static constexpr int kMinWave = 128;
+
 dr_status dr_renderer_create(int32_t wave_paths, dr_renderer **out) try {
     if (!out) return fail(DR_E_ARG, "dr_renderer_create: out is NULL");
     *out = nullptr;
     if (wave_paths < 0) return fail(DR_E_ARG, "dr_renderer_create: negative wave size");
     if (wave_paths == 0) wave_paths = 1 << 22;
-    wave_paths = ((wave_paths + 31) / 32) * 32;
+    // at least kMinWave paths: the photons of one path (16 lights of up to 16) then fit the photon planes of two
+    // records a path, and their lists the extension queue
+    wave_paths = std::max(kMinWave, ((wave_paths + 31) / 32) * 32);
     dr_renderer *r = new (std::nothrow) dr_renderer();
     if (!r) return fail(DR_E_NOMEM, "dr_renderer_create: out of host memory");
     r->capacity = wave_paths;
@@ -1087,9 +1091,10 @@ static cudaError_t ensure_prefix(int *&prefix, int &paths, long long wave) {
     return e;
 }
 
+// Paths a wave may hold: every photon of its paths needs a record (whole warps where that many fit).
 static long long wave_size(const dr_renderer *r, int lights_per_path, long long cap) {
-    long long wave = std::min<long long>(std::min<long long>(r->capacity, cap), (long long)r->shadow_capacity / std::max(1, lights_per_path));
-    return std::max<long long>(32, (wave / 32) * 32);
+    const long long wave = std::min<long long>(std::min<long long>(r->capacity, cap), (long long)r->shadow_capacity / std::max(1, lights_per_path));
+    return wave >= 32 ? wave / 32 * 32 : std::max<long long>(1, wave);
 }
 
 dr_status dr_render_blocks(dr_renderer *r, const dr_scene *sc, const dr_camera *cam, float *fb, int32_t start_block,
