@@ -1163,16 +1163,22 @@ dr_status dr_render_adjoint(dr_renderer *r, const dr_scene *sc, const dr_camera 
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     e = cudaStreamIsCapturing(stream, &capturing);
     if (e != cudaSuccess) return cuda_fail(e, "dr_render_adjoint: stream");
-    const bool direct = capturing != cudaStreamCaptureStatusNone || total <= 1024 + n / 256;
-    if (!direct) {
-        if (r->grad_records < 2 * n) {
-            cudaFree(r->grads);
+    // Without memory for the sums a call does without them.
+    bool direct = capturing != cudaStreamCaptureStatusNone || total <= 1024 + n / 256;
+    if (!direct && r->grad_records < 2 * n) {
+        cudaFree(r->grads);
+        r->grads = nullptr;
+        r->grad_records = 0;
+        e = cudaMalloc((void **)&r->grads, sizeof(float4) * 2 * (size_t)n);
+        if (e == cudaSuccess) r->grad_records = 2 * n;
+        else if (e != cudaErrorMemoryAllocation) return cuda_fail(e, "dr_render_adjoint: gradient sums");
+        else {
+            direct = true;
             r->grads = nullptr;
-            r->grad_records = 0;
-            e = cudaMalloc((void **)&r->grads, sizeof(float4) * 2 * (size_t)n);
-            if (e != cudaSuccess) return cuda_fail(e, "dr_render_adjoint: gradient sums");
-            r->grad_records = 2 * n;
+            (void)cudaGetLastError();
         }
+    }
+    if (!direct) {
         e = drk::load_adjoint_kernels(r->shape);
         if (e == cudaSuccess) e = cudaMemsetAsync(r->grads, 0, sizeof(float4) * 2 * (size_t)n, stream);
         if (e != cudaSuccess) return cuda_fail(e, "dr_render_adjoint: gradient sums");
