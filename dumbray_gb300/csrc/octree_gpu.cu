@@ -441,8 +441,9 @@ inline unsigned blocks(long long n, int t) { return (unsigned)((n + t - 1) / t);
 struct Slab {
     char *p = nullptr;
     size_t bytes = 0, used = 0;
-    explicit Slab(size_t want) {
-        if (want == 0) return;
+    const bool tight;   // no more memory than needed: buffers that grow take no reserve either
+    Slab(size_t want, bool tight_) : tight(tight_) {
+        if (want == 0 || tight) return;
         if (cudaMalloc((void **)&p, want) == cudaSuccess) bytes = want;
         else {
             p = nullptr;
@@ -477,7 +478,7 @@ struct DevBuf {
     T *get(size_t count, Slab *slab = nullptr, size_t guess = 0) {
         const size_t need = std::max<size_t>(count, 1) * sizeof(T);
         if (need > bytes) {
-            const size_t take = bytes ? need + need / 2 : need;
+            const size_t take = bytes && !(slab && slab->tight) ? need + need / 2 : need;
             if (owned) cudaFree(p);
             p = nullptr;
             owned = false;
@@ -512,9 +513,9 @@ struct DevBuf {
     }
 };
 
-}  // namespace
+const char kNoMemory[] = "device allocation failed";
 
-bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, FlatOctree &out, DeviceTree *keep, std::string &err) {
+bool build(const float *xyz, int64_t n, const BuildOptions &opt, FlatOctree &out, DeviceTree *keep, std::string &err, bool tight) {
     out = FlatOctree();
     if (n <= 0) return true;
     if (n >= (int64_t(1) << 31)) {
@@ -546,11 +547,11 @@ bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, Flat
     // about one a triangle.  What a level needs beyond that it allocates; past 4M triangles (2.6 GB here)
     // the allocations no longer show and the guesses would only hold memory.
     const size_t few = (size_t)n + 64, many = 4 * (size_t)n + 1024;
-    Slab slab(n <= (4 << 20) ? many * 49 + few * 284 + 160 * few : 0);
+    Slab slab(n <= (4 << 20) ? many * 49 + few * 284 + 160 * few : 0, tight);
     DevBuf b_xyz, b_refs, b_next, b_owner, b_centre, b_bounds, b_mask, b_off, b_noff, b_sub, b_occ, b_split, b_lbox, b_fc, b_sums, b_tot;
     float *d_xyz = b_xyz.get<float>(9 * (size_t)n);
     int *d_refs = b_refs.get<int>((size_t)n, &slab, many);
-    if (!d_xyz || !d_refs) { err = "device allocation failed"; return false; }
+    if (!d_xyz || !d_refs) { err = kNoMemory; return false; }
     cudaMemcpy(d_xyz, xyz, 36 * (size_t)n, cudaMemcpyHostToDevice);
     k_iota<<<blocks(n, 256), 256>>>(d_refs, (int)n);
 
@@ -569,7 +570,7 @@ bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, Flat
         const int off[2] = {0, (int)n};
         float *d_box = levels[0]->box.get<float>(6, &slab);
         int *d_off = b_off.get<int>(2, &slab, few);
-        if (!d_box || !d_off) { err = "device allocation failed"; return false; }
+        if (!d_box || !d_off) { err = kNoMemory; return false; }
         cudaMemcpy(d_box, b, sizeof(b), cudaMemcpyHostToDevice);
         cudaMemcpy(d_off, off, sizeof(off), cudaMemcpyHostToDevice);
     }
@@ -595,7 +596,7 @@ bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, Flat
         long long *d_first = lv.first.get<long long>(nl, &slab);
         if (!d_owner || !d_centre || !d_sub || !d_mask || !d_occ || !d_split || !d_bounds || !d_lbox || !d_sums || !d_tot || !d_fc ||
             !d_child || !d_count || !d_first) {
-            err = "device allocation failed";
+            err = kNoMemory;
             return false;
         }
         if (nr > 0) {
@@ -633,7 +634,7 @@ bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, Flat
         int *d_noff = b_noff.get<int>((size_t)next->nodes + 1, &slab, few);
         int *d_next = b_next.get<int>((size_t)total.child_refs, &slab, many);
         int *d_leaf = lv.leaf.get<int>((size_t)total.leaf_refs, &slab);
-        if (!d_nbox || !d_noff || !d_next || !d_leaf) { err = "device allocation failed"; return false; }
+        if (!d_nbox || !d_noff || !d_next || !d_leaf) { err = kNoMemory; return false; }
         k_emit<<<blocks(nl, 128), 128>>>(d_sums, d_tot, d_off, d_split, d_occ, d_sub, d_lbox, nl, leaf_total, next_base, d_box, d_child,
                                          d_fc, d_first, d_count, d_noff, d_nbox);
         if (nr > 0) k_leaf_refs<<<blocks(nr, 256), 256>>>(d_sums, d_tot, d_refs, d_owner, d_off, d_split, nr, d_leaf);
@@ -671,7 +672,7 @@ bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, Flat
     int *d_child = b_child.get<int>((size_t)nn), *d_count = b_count.get<int>((size_t)nn);
     long long *d_first = b_first.get<long long>((size_t)nn);
     int *d_leaf = b_leaf.get<int>((size_t)leaf_total);
-    if (!d_lo || !d_hi || !d_child || !d_count || !d_first || !d_leaf) { err = "device allocation failed"; return false; }
+    if (!d_lo || !d_hi || !d_child || !d_count || !d_first || !d_leaf) { err = kNoMemory; return false; }
     cudaError_t e = cudaGetLastError();
     auto copy = [&](void *dst, const void *src, size_t bytes, cudaMemcpyKind kind) {
         if (e == cudaSuccess && bytes) e = cudaMemcpy(dst, src, bytes, kind);
@@ -715,6 +716,17 @@ bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, Flat
         keep->refs = (int32_t *)b_leaf.release();
     }
     return true;
+}
+
+}  // namespace
+
+bool build_octree_gpu(const float *xyz, int64_t n, const BuildOptions &opt, FlatOctree &out, DeviceTree *keep, std::string &err) {
+    if (build(xyz, n, opt, out, keep, err, false)) return true;
+    if (err != kNoMemory) return false;
+    // the slab and the buffers' reserves may be what there was no memory for
+    (void)cudaGetLastError();
+    err.clear();
+    return build(xyz, n, opt, out, keep, err, true);
 }
 
 }  // namespace drb
