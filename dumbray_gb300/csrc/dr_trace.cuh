@@ -10,7 +10,7 @@
 //   * leaf work is shared by the whole warp: the pending (ray, triangle) tests of all lanes that hold
 //     a leaf are numbered by ballots and handed out 32 at a time, one per lane, until none is left;
 //     the tester reads the owner's ray from the warp's shared slots and posts (distance, list
-//     position) to the owner's key with a 64-bit atomicMin, so the owner keeps the smallest distance
+//     position, hit_key) to the owner's key with a 64-bit atomicMin, so the owner keeps the smallest distance
 //     and, among equal distances, the earliest triangle in list order - exactly castInLeaf's
 //     strict-min scan;
 //   * a lane whose ray is finished takes the next ray of the warp's current chunk at once.  Chunks
@@ -38,10 +38,20 @@ enum : int { kIdle = 0, kTrav = 1, kLeaf = 2, kDone = 3 };
 struct WarpSlots {
     float4 o[32];                    // origin, ignored triangle
     float4 d[32];                    // direction, rounding margin of hit points (point_margin)
-    unsigned long long key[32];      // nearest hit of the current leaf: distance bits << 32 | list position
+    unsigned long long key[32];      // nearest hit of the current leaf (hit_key)
     int2 task[32];                   // round's k-th owner: its lane, its first reference - its first task
 };
 constexpr unsigned long long kNoHit = ~0ull;
+
+// A hit as a key whose order is castInLeaf's: the distance (no hit has a negative one), then the list position.
+// Distances are compared as floats there, so -0, which a direction whose product with the normal overflows
+// gives, equals 0: the sign stands below the position.
+__device__ __forceinline__ unsigned long long hit_key(float dist, int pos) {
+    const unsigned b = __float_as_uint(dist);
+    return (unsigned long long)(b & 0x7FFFFFFFu) << 32 | __funnelshift_l(b, (unsigned)pos, 1);
+}
+__device__ __forceinline__ int key_pos(unsigned long long key) { return (int)((unsigned)key >> 1); }
+__device__ __forceinline__ float key_dist(unsigned long long key) { return __uint_as_float((unsigned)(key >> 32) | (unsigned)key << 31); }
 
 struct LaneRay {
     f3 o, inv;                       // counting traversals
@@ -211,8 +221,8 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ty
             h.tri = -1;
             h.t = FLT_MAX;
             if (key != kNoHit) {
-                h.tri = leaf_tri_id(S.leaf_tris, S.leaf_half, (int)(key & 0xFFFFFFFFull));
-                h.t = __uint_as_float((unsigned)(key >> 32));
+                h.tri = leaf_tri_id(S.leaf_tris, S.leaf_half, key_pos(key));
+                h.t = key_dist(key);
                 h.p = xadd(f3of(ws.o[lane]), xmul(f3of(ws.d[lane]), h.t));
             }
             start = src.store(cur_i, h, L.nb, L.nt);
@@ -321,7 +331,7 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ty
                     const float4 o = ws.o[task.x], d = ws.d[task.x];
                     float dist;
                     if (tri_cast(S.leaf_tris, S.leaf_half, pos, f3of(o), f3of(d), clip, __float_as_int(o.w), dist))
-                        atomicMin(&ws.key[task.x], ((unsigned long long)__float_as_uint(dist) << 32) | (unsigned)pos);
+                        atomicMin(&ws.key[task.x], hit_key(dist, pos));
                 }
                 owned += __popc(begins);
             }
@@ -335,7 +345,7 @@ __device__ __forceinline__ void trace_persistent(const Scene &S, Source &src, ty
             mode = kTrav;
             const unsigned long long key = ws.key[lane];
             if (key != kNoHit) {
-                const float t = __uint_as_float((unsigned)(key >> 32));
+                const float t = key_dist(key);
                 const bool occluded = Source::kOccludeBelow > 0.0f && t < Source::kOccludeBelow;
                 const float4 dm = ws.d[lane];
                 const f3 o = f3of(ws.o[lane]), d = f3of(dm), p = xadd(o, xmul(d, t));
