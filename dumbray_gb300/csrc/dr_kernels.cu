@@ -207,8 +207,9 @@ struct BatchSource {
         return true;
     }
     __device__ __forceinline__ bool load(int i, f3 &ro, f3 &rd, int &ign, int &job) {
-        ro = mkf3(o[3 * i], o[3 * i + 1], o[3 * i + 2]);
-        rd = mkf3(d[3 * i], d[3 * i + 1], d[3 * i + 2]);
+        const size_t at3 = 3 * (size_t)i;   // past 2^31 from 0.72e9 rays on
+        ro = mkf3(o[at3], o[at3 + 1], o[at3 + 2]);
+        rd = mkf3(d[at3], d[at3 + 1], d[at3 + 2]);
         ign = ignore ? ignore[i] : -1;
         job = 0;
         return true;
