@@ -137,8 +137,9 @@ static __device__ __noinline__ bool exact_slab(f3 l, f3 h, f3 o, f3 d) {
     const f3 inv = mkf3(__fdiv_rn(1.0f, d.x), __fdiv_rn(1.0f, d.y), __fdiv_rn(1.0f, d.z));
     return slab_hit(l.x, l.y, l.z, h.x, h.y, h.z, o, inv, true);
 }
-// Bounds what rounding does to a hit point (2 u (|o| + 2 reach)) and to the plane distances of a box of
-// the scene (2.1 u (|x| + |o|) in space), three times over.
+// Bounds what rounding does to a hit point in a box of the scene (d t, then the sum: u (|o| + 2 reach),
+// u = 2^-24), to the plane distances of that box (three roundings: 3 u (|o| + reach) in space) and to the
+// comparison with the face (u reach): u (4 |o| + 6 reach) in all, more than twice over.
 __device__ __forceinline__ float point_margin(f3 o, float reach) { return 9.5367431640625e-7f * (fabsf(o.x) + fabsf(o.y) + fabsf(o.z) + reach); }   // 2^-20
 
 // Two floats in one register pair, and operations on both (one issue slot on sm_100 and later), each
@@ -338,10 +339,11 @@ constexpr int kCountShift = 11;
 // sign of the direction (no min / max of the pair), with one fused multiply-add each.
 //   exact, per plane:  t = rn(rn(x - o) * inv), inv = rn(1 / d)
 //   here:              t = rn(x' * inv - off), off = rn(o * inv) -+ slack
-// Rounding separates the two by at most 5.2 u |x| |inv| + 7.2 u |o| |inv| (u = 2^-24; 2 of each for the
-// approximate reciprocal here).  The planes are
-// widened by 2^-19 x reach >= 32 u |x| and the offsets by 2^-20 |o inv| = 16 u |o| |inv|, six times and
-// twice that; the far offset also takes 2 kEps for the exact test's kEps on either end.
+// Rounding separates the two by at most 7 u |x| |inv| + 8 u |o| |inv| (u = 2^-24).  Of each, 3 are the exact
+// test's difference, product and reciprocal, 2 the approximate reciprocal here and 1 the fused operation; the
+// last of |x| is the widened plane's rounding, the last two of |o| those of o * inv and of the offset.  The
+// planes are widened by 2^-19 x reach >= 32 u |x| and the offsets by 2^-20 |o inv| = 16 u |o| |inv|, four times
+// and twice that; the far offset also takes 2 kEps for the exact test's kEps on either end.
 // What bounds it is instruction issue (55-69% of the issue slots at 15-17 of 32 lanes) and the wait for
 // the record; against the exact test on nodes and planes, in one call: 8.4M incoherent casts on the
 // 1.31M-triangle mesh 5.02 -> 4.34 ms, the 1080p 16 spp path trace 48.9 -> 44.2 ms, the room of 20k

@@ -12,6 +12,8 @@
 //                     in the adjoint pass it also scatters gradients of emission hits
 //   k_shadow_phys     point -> light visibility; in the adjoint pass it marks the visible records
 //   k_adj_shadow      adjoint pass: gradients of the visible NEE contributions
+//   k_add_gradients   adjoint pass: a call's gradient sums to the caller's arrays
+//   k_scene_*, k_leaf_tris, k_group_records   scene records from a built tree; k_rebase_* their batch copies
 //   k_resolve         accumulators -> BlockBasedFrameBuffer<8,16> set / blend (BlockBasedFrameBuffer.impl.cuh:149-156)
 //
 // Wavefront design: queues are structure-of-arrays of float4/int4 records in HBM; work is pulled by
@@ -305,7 +307,7 @@ struct WaveArgs {
     Queue q[2];
     float2 *hits;
     ShadowQ sq;
-    ShadowQ cq;             // carry region of the shadow planes (blocked reference photons)
+    ShadowQ cq;             // carry region of the shadow planes (reference photons between two casts)
     int carry_cap, shadow_cap;
     bool roomy;             // the carry region holds every photon of the wave
     float *accum;           // [total slots][4]
@@ -496,7 +498,8 @@ struct TraceSource {
 };
 
 // Block shape of the traversal kernels (k_trace, k_shadow_phys, k_shadow_ref): 8 warps, 4 blocks per SM
-// cap registers at 64 (32 warps per SM), which the traversal state fits without spilling.  4 against 3
+// cap registers at 64 (32 warps per SM), which the traversal state fits but for 4 bytes of spills (12 in
+// k_shadow_ref, 12-20 in k_cast).  4 against 3
 // blocks (80 registers), in one call: room 9.40 -> 8.67 ms, 1080p photon render 44.2 -> 42.1 ms, path
 // trace 38.4 -> 35.7 ms, gradients 73.0 -> 70.4 ms.  The counting instances hold boxes and counts as well and
 // spill 126 bytes at 64 registers; 3 blocks (80 registers): 256^2 x 4 counted renders 3.04 -> 2.86 ms in the
@@ -894,7 +897,7 @@ __device__ __forceinline__ void scatter_albedo(const Item &I, const int *pre, in
 }
 
 // Physical path step.  ADJ: adjoint pass (no image; gradients of emission hits are scattered here,
-// vertex triangles are recorded for the NEE gradients scattered by k_shadow_phys).
+// vertex triangles are recorded for the NEE gradients scattered by k_adj_shadow).
 template <bool MULTI, bool ADJ>
 __global__ void __launch_bounds__(kShadeThreads, kShadePhysBlocksPerSM) k_shade_phys(WaveArgs A, int b) {
     Ctrl *C = A.ctrl;

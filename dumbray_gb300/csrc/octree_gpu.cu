@@ -15,6 +15,9 @@
 //       where each split node's children and each leaf's list go (breadth-first order),
 //   (8) the next level's nodes and, for every split node, its references copied to the lists of the
 //       octants they overlap, in list order (a warp per node, the block for large ones).
+// Staging the sums of (3), a thread per octant in (4) and the block's part in (8) took a scene of 82k triangles
+// (displaced icosphere, physical padding, split 4) from 22.2 to 18.6 ms and one of 1.31M from 352 to 297 ms; what
+// the later steps gave stands at their kernels.
 // After the last level inner boxes shrink to their children's, level by level from the deepest.  The
 // host reads three totals a level (sizes of the next level's arrays) and the finished tree.  All geometry
 // comes from octree_geom.h; nvcc compiles it with -fmad=false and IEEE division / square root, the host
@@ -130,8 +133,6 @@ __global__ void __launch_bounds__(32 * kStageWarps) k_split_points(const float *
     for (int i = 0; i < 8; i++) store_box(sub, 8 * k + i, o[i]);
 }
 
-// Same call, scenes of the displaced icosphere, physical padding, split 4: with these three kernels
-// (sums, masks, lists) 82k triangles 22.2 -> 18.6 ms, 1.31M triangles 352 -> 297 ms.
 // Octant overlap of every reference: a thread per (reference, octant), the mask byte from a ballot.
 // (One thread per reference took its eight tests one after another, each as long as the longest of the
 // warp's.  Gathering a block's clipped pairs before clipping them was slower than both.)

@@ -340,7 +340,7 @@ void dr_renderer_destroy(dr_renderer *r);
  * pipeline's kernels fill the tails of another's (the reference runs several GPU worker threads
  * per device for the same reason, Renderer::ThreadConfiguration).  Each extra lane allocates a
  * scratch set like the renderer's own on first use.  Results do not depend on the lane count
- * beyond float accumulation order.  Batches and the adjoint use one lane. */
+ * beyond float accumulation order.  Batches (graphs too) and the adjoint use the lanes as well. */
 #define DR_DEFAULT_LANES 4
 #define DR_MAX_LANES 8
 dr_status dr_renderer_set_lanes(dr_renderer *r, int32_t lanes);
@@ -348,7 +348,7 @@ int32_t dr_renderer_lanes(const dr_renderer *r);
 
 /* Block shape of the traversal kernels (no counterpart in the reference, which launches one
  * thread per pixel): 0 = 256 threads x 4 blocks per SM (default), 1 = 128 threads x 8 blocks per SM.
- * Both cap registers at 80 and keep the same threads in flight; they differ in how warps share an
+ * Both cap registers at 64 and keep the same threads in flight; they differ in how warps share an
  * SM's blocks and leave the tail of a launch.  Results do not depend on the shape.  A batch graph
  * captured with one shape is re-captured when the renderer's shape changes. */
 dr_status dr_renderer_set_block_shape(dr_renderer *r, int32_t shape);
